@@ -58,7 +58,10 @@ extern "C" {
                          /* 0.01 A recomputed exactly in FP64; error <= 1e-4 A        */
 #define WMD_MODE_I8X2 2  /* 2 limbs (16-bit fixed point), all 4 products, exact Gram  */
                          /* matrix of the quantised frames; error ~2e-4 A             */
-#define WMD_MODE_FP64 3  /* FP64 SIMT covariance tiles (accuracy reference on GPU)    */
+#define WMD_MODE_FP64 3  /* FP64-accurate (accuracy reference on GPU): 40-bit fixed   */
+                         /* point per frame on the tensor cores, pairs too close for  */
+                         /* it recomputed in FP64; FP64 SIMT tiles for small matrices */
+                         /* and for over 26,176 atoms                                 */
 
 /* Per-frame statistics written by wmd_rmsd_forward and read by
  * wmd_rmsd_backward: 16 doubles per frame
@@ -168,7 +171,7 @@ int wmd_pairwise_rmsd(wmd_ctx* ctx, const float* coords, int64_t n_frames, int64
  * (the tile partition of PairwiseRmsdPlan::finalize's i < j loop,
  * plan.rs:593-674, which the reference runs as one loop).  Every caller holds
  * all frames; part `part` computes the pairs i < j whose tile row (40 frames
- * in the tensor-core modes, 32 in the SIMT modes) is part (mod parts), writes
+ * on the tensor cores, 32 on the SIMT tiles) is part (mod parts), writes
  * each at (i, j) and (j, i), and leaves every other entry 0.  The parts for
  * part = 0..parts-1 are disjoint and their sum is wmd_pairwise_rmsd's matrix
  * exactly (the tensor-core modes quantise every frame with the same

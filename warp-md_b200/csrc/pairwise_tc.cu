@@ -60,6 +60,7 @@
 #include "device_util.cuh"
 #include "pairwise_tc.h"
 #include "qcp.cuh"
+#include "tcgen05.cuh"
 
 namespace wmd {
 namespace {
@@ -109,100 +110,11 @@ struct TcGeo {
 // Pairs whose truncated 3-limb RMSD falls below this are recomputed exactly.
 constexpr float kRefineRmsd = 0.01f;
 
-// ------------------------------------------------------------------ PTX --
-
-__device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, int ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(dst_smem)),
-               "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, int ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// 32 lanes x 8 consecutive 32-bit TMEM columns -> 8 registers per thread
-// (call tmem_wait_ld before using them)
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int32_t* v) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-      "[%5];" ::"r"(smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
-      : "memory");
-}
-
-// Shared-memory matrix descriptor, K-major, rows of ROW bytes with the
-// matching swizzle (64: SWIZZLE_64B, layout 4; 32: SWIZZLE_32B, layout 6),
-// 8-row core groups 8 ROW bytes apart, sm_100 descriptor version 1.
-template <int ROW>
-__device__ __forceinline__ uint64_t desc_sw(const void* p) {
-  static_assert(ROW == 32 || ROW == 64, "row bytes");
-  const uint64_t start = (smem_addr(p) >> 4) & 0x3FFFu;
-  return start | (uint64_t(1) << 16) | (uint64_t((8 * ROW) >> 4) << 32) | (uint64_t(1) << 46) |
-         (uint64_t(ROW == 64 ? 4 : 6) << 61);
-}
-
 // kind::i8 instruction descriptor: D s32, A/B s8, both K-major, M=128, N=96.
 constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(kTileN >> 3) << 17) |
                             (uint32_t(kTileM >> 4) << 24);
 
-// bounded wait on an mbarrier phase (no shared abort fallback needed by
-// callers other than through the flag)
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, int* status, volatile int* abort,
-                                        uint64_t limit_ns) {
-  return mbar_wait(bar, parity, status, kStatusTimeoutFull, abort, limit_ns);
-}
-
-// Tiles are enumerated in groups of kRowGroup tile rows, column after column
-// inside a group, so that the ~148 tiles in flight at once share a few A rows
-// and B columns and their limbs stay in L2.  (Row after row, they would share
-// one A row but stream 148 B columns, rereading each column from DRAM for
-// every row once the limbs outgrow L2: 196 MB for 20,000 frames x 1,000 atoms.)
-constexpr int kRowGroup = 8;
-
-struct TileList {
-  int ni, nj;  // I blocks (40 frames) x J blocks (40 frames)
-  int64_t F;
-  int part, parts;  // this launch computes the I blocks bi = part (mod parts)
-  __device__ __forceinline__ bool valid(int64_t t, int& bi, int& bj) const {
-    const int64_t gsz = (int64_t)kRowGroup * nj;
-    const int64_t g = t / gsz, r = t - g * gsz;
-    const int rows = min(kRowGroup, ni - (int)g * kRowGroup);
-    bj = (int)(r / rows);
-    bi = (int)g * kRowGroup + (int)(r - (int64_t)bj * rows);
-    if (bi % parts != part) return false;
-    const int64_t i0 = (int64_t)bi * kTileFramesM;
-    const int64_t jmax = min((int64_t)(bj + 1) * kTileFramesN, F) - 1;
-    return i0 < jmax && (int64_t)bj * kTileFramesN < F;  // some pair i < j in the tile
-  }
-};
+using PairTiles = TileWalk<kTileFramesM, kTileFramesN>;
 
 struct TcArgs {
   int64_t F;
@@ -225,7 +137,7 @@ struct TcArgs {
 template <int LIMBS>
 __global__ void __launch_bounds__(kTcThreads, 1)
     pair_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                   const TcArgs args, const TileList tiles) {
+                   const TcArgs args, const PairTiles walk, int64_t n_tiles) {
   using G = TcGeo<LIMBS>;
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int kStagesTc = G::kStages;
@@ -240,7 +152,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_k = (int)(args.n_pad / G::kKChunk);
-  const int64_t n_tiles = (int64_t)tiles.ni * tiles.nj;
+  PairTiles tiles = walk;  // every role walks its own cursor
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStagesTc; ++s) {
@@ -268,7 +180,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       bool ok = true;
       for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
         int bi, bj;
-        if (!tiles.valid(t, bi, bj)) continue;
+        if (!tiles.at(t, bi, bj)) continue;
         for (int kc = 0; kc < n_k; ++kc, ++it) {
           const int s = it % kStagesTc;
           const uint32_t ph = (it / kStagesTc) & 1u;
@@ -298,7 +210,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const uint64_t dbase = desc_sw<G::kKChunk>(smem);
       for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
         int bi, bj;
-        if (!tiles.valid(t, bi, bj)) continue;
+        if (!tiles.at(t, bi, bj)) continue;
         // the epilogue must have drained the previous tile's accumulators
         if (!tc_wait(tmem_empty, (tc & 1u) ^ 1u, args.status, abort_flag, args.wait.limit_ns)) { ok = false; break; }
         tc_fence_after();
@@ -362,7 +274,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     uint32_t tc = 0;
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
       int bi, bj;
-      if (!tiles.valid(t, bi, bj)) continue;
+      if (!tiles.at(t, bi, bj)) continue;
       if (drainer) {
         if (tc_wait(tmem_full, tc & 1u, args.status, abort_flag, args.wait.limit_ns)) {
           tc_fence_after();
@@ -575,19 +487,21 @@ __global__ void __launch_bounds__(256) tc_prep_limbs(const float* __restrict__ c
   }
 }
 
-// 3 limbs: pairs whose truncated RMSD came out below kRefineRmsd, recomputed
-// exactly in FP64 from the coordinates, a warp per pair: the centred sums H,
+// The pairs the tensor-core epilogues listed (3 limbs: RMSD below kRefineRmsd;
+// the 40-bit form: see pairwise_tc64.cu), recomputed in FP64 from the coordinates, a warp per pair: the centred sums H,
 // G_i, G_j and QCP (metric rms), or sum |x_i - x_j|^2 (nofit), each lane
 // taking atoms lane, lane + 32, ... and the warp adding its lanes in a fixed
-// tree.  When more pairs were flagged than the list holds, every pair (i, j),
+// tree.  When more pairs were flagged than the list holds, nothing is done
+// here (scan 0: the caller recomputes the whole matrix), or every pair (i, j),
 // i < j, of this launch's tile rows (i / 40 = part mod parts) whose entry is
-// below kRefineRmsd is found in the matrix itself.
+// below kRefineRmsd is found in the matrix itself (scan 1).
 __global__ void __launch_bounds__(256) pair_refine_kernel(const float* __restrict__ coords, int64_t n_atoms, int stride,
                                                           const uint32_t* __restrict__ sel, int64_t n_sel, int64_t F,
                                                           const double* __restrict__ cen, int metric,
                                                           const uint2* __restrict__ list,
                                                           const unsigned* __restrict__ count, unsigned cap,
-                                                          float* __restrict__ out, int part, int parts, int* status) {
+                                                          float* __restrict__ out, int part, int parts, int scan,
+                                                          int* status) {
   const int lane = threadIdx.x & 31;
   const int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -642,6 +556,7 @@ __global__ void __launch_bounds__(256) pair_refine_kernel(const float* __restric
     for (int64_t p = wg; p < (int64_t)n_list; p += nw) refine(list[p].x, list[p].y);
     return;
   }
+  if (!scan) return;
   for (int64_t i = wg; i < F; i += nw) {
     if ((int)((i / kTileFramesM) % parts) != part) continue;
     for (int64_t j0 = i + 1; j0 < F; j0 += 32) {
@@ -677,6 +592,38 @@ EncodeTiled encode_fn(std::string* msg) {
   fn = reinterpret_cast<EncodeTiled>(p);
   return fn;
 }
+
+}  // namespace
+
+cudaError_t launch_pair_refine(const PairFlags& flags, int sm_count, const float* coords, int64_t n_atoms, int stride,
+                               const uint32_t* sel, int64_t n_sel, int64_t F, int metric, float* out, int part,
+                               int parts, bool scan, int* status, cudaStream_t s) {
+  pair_refine_kernel<<<(unsigned)(2 * sm_count), 256, 0, s>>>(coords, n_atoms, stride, sel, n_sel, F, flags.cen, metric,
+                                                               flags.list, flags.count, flags.cap, out, part, parts,
+                                                               scan ? 1 : 0, status);
+  return cudaGetLastError();
+}
+
+// The digit array L[limb][row][k] as a 3-D map whose box is one stage operand:
+// `chunk` atoms x `tile_rows` rows x all limbs, swizzled to the box row.
+int encode_digits(CUtensorMap* map, const int8_t* digits, int64_t n_pad, int64_t rows, int limbs, int chunk,
+                  int tile_rows, std::string* msg) {
+  EncodeTiled enc = encode_fn(msg);
+  if (!enc) return WMD_ERR_CUDA;
+  const cuuint64_t dims[3] = {(cuuint64_t)n_pad, (cuuint64_t)rows, (cuuint64_t)limbs};
+  const cuuint64_t strides[2] = {(cuuint64_t)n_pad, (cuuint64_t)(rows * n_pad)};
+  const cuuint32_t box[3] = {(cuuint32_t)chunk, (cuuint32_t)tile_rows, (cuuint32_t)limbs};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(digits), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         chunk == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r == CUDA_SUCCESS) return 0;
+  *msg = "cuda driver error: cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
+  return WMD_ERR_CUDA;
+}
+
+namespace {
 
 template <int LIMBS>
 int run_tc(PairwiseWorkspace& w, int sm_count, const float* coords, int64_t F, int64_t n_atoms, int stride,
@@ -728,26 +675,10 @@ int run_tc(PairwiseWorkspace& w, int sm_count, const float* coords, int64_t F, i
     return WMD_ERR_CUDA;
   }
 
-  EncodeTiled enc = encode_fn(msg);
-  if (!enc) return WMD_ERR_CUDA;
   CUtensorMap map_a, map_b;
-  const cuuint64_t dims[3] = {(cuuint64_t)n_pad, (cuuint64_t)rows_pad, (cuuint64_t)LIMBS};
-  const cuuint64_t strides[2] = {(cuuint64_t)n_pad, (cuuint64_t)(rows_pad * n_pad)};
-  const cuuint32_t box_a[3] = {G::kKChunk, kTileM, LIMBS};
-  const cuuint32_t box_b[3] = {G::kKChunk, kTileN, LIMBS};
-  const CUtensorMapSwizzle swz = G::kKChunk == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
-  const cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(&map_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, limbs, dims, strides, box_a, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r == CUDA_SUCCESS)
-    r = enc(&map_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, limbs, dims, strides, box_b, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    *msg = "cuda driver error: cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
-    return WMD_ERR_CUDA;
-  }
+  int rc = encode_digits(&map_a, limbs, n_pad, rows_pad, LIMBS, G::kKChunk, kTileM, msg);
+  if (!rc) rc = encode_digits(&map_b, limbs, n_pad, rows_pad, LIMBS, G::kKChunk, kTileN, msg);
+  if (rc) return rc;
 
   TcArgs a;
   a.F = F;
@@ -763,28 +694,28 @@ int run_tc(PairwiseWorkspace& w, int sm_count, const float* coords, int64_t F, i
   a.flagged = flagged;
   a.n_flagged = n_flagged;
   a.cap = cap;
-  TileList tl;
-  tl.ni = (int)((F + kTileFramesM - 1) / kTileFramesM);
-  tl.nj = (int)((F + kTileFramesN - 1) / kTileFramesN);
-  tl.F = F;
-  tl.part = w.part;
-  tl.parts = w.parts;
+  const PairTiles tl(F, w.part, w.parts);
   auto kern = pair_tc_kernel<LIMBS>;
   if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmemBytes)) != cudaSuccess) {
     *msg = std::string("cuda driver error: ") + cudaGetErrorString(e);
     return WMD_ERR_CUDA;
   }
-  const int64_t n_tiles = (int64_t)tl.ni * tl.nj;
+  const int64_t n_tiles = tl.count();
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count, n_tiles));
-  kern<<<grid, kTcThreads, G::kSmemBytes, s>>>(map_a, map_b, a, tl);
+  kern<<<grid, kTcThreads, G::kSmemBytes, s>>>(map_a, map_b, a, tl, n_tiles);
   if ((e = cudaGetLastError()) != cudaSuccess) {
     *msg = std::string("cuda driver error: pairwise tensor-core launch: ") + cudaGetErrorString(e);
     return WMD_ERR_CUDA;
   }
   if (G::kShift) {
-    pair_refine_kernel<<<(unsigned)(2 * sm_count), 256, 0, s>>>(coords, n_atoms, stride, sel, n_sel, F, cen, metric,
-                                                                 flagged, n_flagged, cap, out, w.part, w.parts, status);
-    if ((e = cudaGetLastError()) != cudaSuccess) {
+    PairFlags flags;
+    flags.list = flagged;
+    flags.count = n_flagged;
+    flags.cap = cap;
+    flags.cen = cen;
+    e = launch_pair_refine(flags, sm_count, coords, n_atoms, stride, sel, n_sel, F, metric, out, w.part, w.parts, true,
+                           status, s);
+    if (e != cudaSuccess) {
       *msg = std::string("cuda driver error: pairwise refine launch: ") + cudaGetErrorString(e);
       return WMD_ERR_CUDA;
     }

@@ -183,6 +183,15 @@ WMD_HD QcpOut qcp_lambda(const double h[9], double e0) {
 
 
 
+// Quotient for a Newton step: the next iteration corrects its last bits.
+WMD_HD float newton_quotient(float a, float b) {
+#if defined(__CUDA_ARCH__)
+  return __fdividef(a, b);
+#else
+  return a / b;
+#endif
+}
+
 // Mean-square deviation of a frame pair in the tensor-core epilogue, with as
 // little FP64 arithmetic as the cancellation allows (on sm_100a FP64 issue
 // stalls beside tensor-core MMAs, FP32 does not).  H (9 entries) is exact in
@@ -251,7 +260,7 @@ WMD_HD bool qcp_msd_mixed(const long long hq[9], double gx, double gy, float n, 
     const float q = (((u - 4.0f) * u + b2) * u + b1) * u + b0;
     dq = ((4.0f * u - 12.0f) * u + 2.0f * b2) * u + b1;
     if (!(dq != 0.0f)) break;
-    const float du = q / dq;
+    const float du = newton_quotient(q, dq);
     u -= du;
     if (fabsf(du) <= 2e-7f * fabsf(u) + 1e-30f) {
       converged = true;
@@ -266,6 +275,77 @@ WMD_HD bool qcp_msd_mixed(const long long hq[9], double gx, double gy, float n, 
   if (!converged || !(fabsf(dq) > 1e-2f) || !(u == u)) return false;
   const float mm = (float)D * u / n * s2;
   *msd = mm > 0.0f ? mm : 0.0f;
+  return true;
+}
+
+// sum |x_i - R x_j|^2 = D - 2 lambda_max of a frame pair at FP64 accuracy, for the
+// exact-integer tensor-core epilogue: h the nine covariance sums, D = G_x + G_y,
+// all in one unit.  The same shifted quartic as qcp_msd_mixed (u = 1 -
+// lambda_max / e0, e0 = D / 2), with every coefficient in FP64 from H / e0; the
+// search for the root runs in FP32 to its last bits, and an FP64 Newton step on
+// the FP64 coefficients follows (more while one moves u by over 1e-7 |slope| of
+// itself): it leaves that times the FP32 slope's error, ~1e-6 / |slope|.  About
+// 95 FP64 operations a pair against 190 and a division per iteration for
+// qcp_lambda, which matters because FP64 issue stalls beside tensor-core MMAs.
+// Returns false, leaving *gap unset, where the root is not clearly simple or D
+// is out of the FP32 range (the caller takes qcp_lambda).
+WMD_HD bool qcp_gap(const double h[9], double D, double* gap) {
+  if (!(D > 1e-30 && D < 1e30)) return false;
+  // w = 1 / e0 from the FP32 quotient by two Newton-Raphson steps
+  const double e0 = 0.5 * D;
+  double w = (double)(1.0f / (float)e0);
+  w += w * (1.0 - e0 * w);
+  w += w * (1.0 - e0 * w);
+  double a[9];
+  for (int i = 0; i < 9; ++i) a[i] = h[i] * w;
+  double ss = 0.0;
+  for (int i = 0; i < 9; ++i) ss += a[i] * a[i];
+  const double d2 = -2.0 * ss, d1 = -8.0 * det3(a);
+  const double b2 = 6.0 + d2, b1 = -(4.0 + 2.0 * d2 + d1);
+  // M = I - K / e0, symmetric
+  const double p = a[0] + a[4], q = a[0] - a[4], lo = 1.0 - a[8], hi = 1.0 + a[8];
+  const double m00 = lo - p, m11 = hi - q, m22 = hi + q, m33 = lo + p;
+  const double m01 = a[7] - a[5], m02 = a[2] - a[6], m03 = a[3] - a[1];
+  const double m12 = -(a[1] + a[3]), m13 = -(a[2] + a[6]), m23 = -(a[5] + a[7]);
+  const double c5 = m22 * m33 - m23 * m23, c4 = m12 * m33 - m23 * m13, c3 = m12 * m23 - m22 * m13;
+  const double c2 = m02 * m33 - m23 * m03, c1 = m02 * m23 - m22 * m03, c0 = m02 * m13 - m12 * m03;
+  double b0 = (m00 * m11 - m01 * m01) * c5;
+  b0 -= (m00 * m12 - m02 * m01) * c4;
+  b0 += (m00 * m13 - m03 * m01) * c3;
+  b0 += (m01 * m12 - m02 * m11) * c2;
+  b0 -= (m01 * m13 - m03 * m11) * c1;
+  b0 += (m02 * m13 - m03 * m12) * c0;
+  const float f0 = (float)b0, f1 = (float)b1, f2 = (float)b2;
+  float uf = 0.0f;
+  bool converged = false;
+  for (int it = 0; it < 24; ++it) {
+    const float qv = (((uf - 4.0f) * uf + f2) * uf + f1) * uf + f0;
+    const float dq = ((4.0f * uf - 12.0f) * uf + 2.0f * f2) * uf + f1;
+    if (!(dq != 0.0f)) break;
+    const float du = newton_quotient(qv, dq);
+    uf -= du;
+    if (fabsf(du) <= 2e-7f * fabsf(uf) + 1e-30f) {
+      converged = true;
+      break;
+    }
+  }
+  const float slope = ((4.0f * uf - 12.0f) * uf + 2.0f * f2) * uf + f1;
+  if (!converged || !(fabsf(slope) > 1e-2f)) return false;
+  const float inv_slope = 1.0f / slope;
+  const float tiny = 1e-7f * fabsf(uf) * fminf(10.0f, fabsf(slope)) + 1e-30f;
+  double u = (double)uf;
+  bool settled = false;
+  for (int it = 0; it < 6; ++it) {
+    const double qv = (((u - 4.0) * u + b2) * u + b1) * u + b0;
+    const float du = (float)qv * inv_slope;
+    u -= (double)du;
+    if (fabsf(du) <= tiny) {
+      settled = true;
+      break;
+    }
+  }
+  if (!settled) return false;
+  *gap = u > 0.0 ? D * u : 0.0;
   return true;
 }
 
