@@ -29,6 +29,7 @@
 #ifndef WARPMD_RMSD_H
 #define WARPMD_RMSD_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -90,6 +91,16 @@ const char* wmd_version(void);
  * (crates/traj-gpu/src/cuda/runtime_core.rs:127-137). */
 int wmd_reference_upload(wmd_ctx* ctx, const float* ref, int64_t n_sel, int stride, wmd_ref** out);
 int wmd_reference_free(wmd_ctx* ctx, wmd_ref* ref);
+/* The same for a reference in device memory, centred on the device by a kernel
+ * on `stream`: no copy, allocation or host synchronization, so it can be
+ * captured in a CUDA graph.  The centred coordinates live in the caller's
+ * `workspace` (device memory, 256-byte aligned, wmd_reference_workspace(n_sel)
+ * bytes), which must outlive the wmd_ref and every call enqueued with it; work
+ * on another stream must be ordered after `stream`.  wmd_reference_free does
+ * not free the workspace. */
+size_t wmd_reference_workspace(int64_t n_sel);
+int wmd_reference_prepare(wmd_ctx* ctx, const float* ref, int64_t n_sel, int stride, void* workspace,
+                          size_t workspace_bytes, void* stream, wmd_ref** out);
 
 /* Error-path diagnostics (no counterpart in the reference, whose CUDA failures
  * surface as TrajError::Unsupported, crates/traj-gpu/src/cuda.rs:384-390).

@@ -342,18 +342,26 @@ int pairwise_run(PairwiseWorkspace& w, int sm_count, const float* coords, int64_
     w.frames_cap = n_frames;
   }
   Guard guard;
-  if (tc64) {
+  bool on_tc = tc64;
+  if (on_tc) {
     PairFlags flags;
-    if ((rc = pairwise_tc64_run(w, sm_count, coords, n_frames, n_atoms, stride, sel, n_sel, metric, out, status, s, msg,
-                                &flags)))
+    rc = pairwise_tc64_run(w, sm_count, coords, n_frames, n_atoms, stride, sel, n_sel, metric, out, status, s, msg,
+                           &flags);
+    if (rc == WMD_ERR_OOM) {  // no room for the digits beside the panels: the SIMT tiles need none
+      on_tc = false;
+      if ((e = cudaMemsetAsync(out, 0, (size_t)n_frames * n_frames * sizeof(float), s)) != cudaSuccess)
+        return cuda_fail(e, "");
+    } else if (rc) {
       return rc;
-    if ((e = launch_pair_refine(flags, sm_count, coords, n_atoms, stride, sel, n_sel, n_frames, metric, out, w.part,
-                                w.parts, false, status, s)) != cudaSuccess)
-      return cuda_fail(e, "pairwise refine launch: ");
-    guard.count = flags.count;
-    guard.cap = flags.cap;
+    } else {
+      if ((e = launch_pair_refine(flags, sm_count, coords, n_atoms, stride, sel, n_sel, n_frames, metric, out, w.part,
+                                  w.parts, false, status, s)) != cudaSuccess)
+        return cuda_fail(e, "pairwise refine launch: ");
+      guard.count = flags.count;
+      guard.cap = flags.cap;
+    }
   }
-  const int row_frames = tc64 ? 40 : kPanelFrames;
+  const int row_frames = on_tc ? 40 : kPanelFrames;
   e = f64 ? run_simt<double>(w, sm_count, coords, n_frames, n_atoms, stride, sel, n_sel, n_pad, metric, row_frames,
                              guard, out, status, s)
           : run_simt<float>(w, sm_count, coords, n_frames, n_atoms, stride, sel, n_sel, n_pad, metric, row_frames,

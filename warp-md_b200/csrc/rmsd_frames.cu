@@ -81,9 +81,9 @@ __device__ __noinline__ void finish_frame(const FrameLaunch& L, int64_t f, doubl
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) h[a * 3 + b] = tot[6 + a * 3 + b] - sx[a] * L.ref.sum_c[b] * inv_n;
+    for (int b = 0; b < 3; ++b) h[a * 3 + b] = tot[6 + a * 3 + b] - sx[a] * ref_sum_c(L.ref, b) * inv_n;
   const double gx = sxx - (sx[0] * sx[0] + sx[1] * sx[1] + sx[2] * sx[2]) * inv_n;
-  const double gy = L.ref.gy;
+  const double gy = ref_gy(L.ref);
   const QcpOut q = qcp_lambda(h, 0.5 * (gx + gy));
   const double rmsd = sqrt(msd_from(gx, gy, q.lambda, n));
   if (L.out.rmsd) L.out.rmsd[f] = rmsd;
@@ -218,6 +218,8 @@ __global__ void __launch_bounds__(kThreads, 3) rmsd_frames_kernel(const FrameLau
     }
   }
 
+  const double mean[3] = {MODE == kFwdRaw ? ref_mean(L.ref, 0) : 0.0, MODE == kFwdRaw ? ref_mean(L.ref, 1) : 0.0,
+                          MODE == kFwdRaw ? ref_mean(L.ref, 2) : 0.0};
   double yr[APT][3];
   float wr[MODE == kFwdW ? APT : 1];
   uint32_t gidx[GATHER ? APT : 1];
@@ -342,9 +344,9 @@ __global__ void __launch_bounds__(kThreads, 3) rmsd_frames_kernel(const FrameLau
           float x0, x1, x2;
           load_x(j, x0, x1, x2);
           // y = y_c + mean, rebuilt in FP64; x - y in FP64
-          const double d0 = (double)x0 - (yr[j][0] + L.ref.mean[0]);
-          const double d1 = (double)x1 - (yr[j][1] + L.ref.mean[1]);
-          const double d2 = (double)x2 - (yr[j][2] + L.ref.mean[2]);
+          const double d0 = (double)x0 - (yr[j][0] + mean[0]);
+          const double d1 = (double)x1 - (yr[j][1] + mean[1]);
+          const double d2 = (double)x2 - (yr[j][2] + mean[2]);
           const bool in = ok && tid + j * kConsumerThreads < len;
           acc[0] = fma(d0, in ? d0 : 0.0, acc[0]);
           acc[1] = fma(d1, in ? d1 : 0.0, acc[1]);
@@ -445,7 +447,8 @@ __global__ void __launch_bounds__(256) rmsd_refine_kernel(const FrameLaunch L) {
     double R[9], c[3];
     for (int e = 0; e < 9; ++e) R[e] = sh_r[e];
     c[0] = sh_r[9]; c[1] = sh_r[10]; c[2] = sh_r[11];
-    const double my0 = L.ref.sum_c[0] * inv_n, my1 = L.ref.sum_c[1] * inv_n, my2 = L.ref.sum_c[2] * inv_n;
+    const double my0 = ref_sum_c(L.ref, 0) * inv_n, my1 = ref_sum_c(L.ref, 1) * inv_n,
+                 my2 = ref_sum_c(L.ref, 2) * inv_n;
     const float* frame = L.coords + (size_t)f * L.n_atoms * STRIDE;
     double acc = 0.0;
     for (int64_t k = threadIdx.x; k < n_sel; k += blockDim.x) {
@@ -508,6 +511,8 @@ __global__ void __launch_bounds__(kGatherThreads) rmsd_gather_kernel(const Frame
   const int n_tiles = (int)((n_sel + tile - 1) / tile);
   const int64_t W = (int64_t)n_tiles * F;
   const int64_t w0 = W * gw / n_warps, w1 = W * (gw + 1) / n_warps;
+  const double mean[3] = {MODE == kFwdRaw ? ref_mean(L.ref, 0) : 0.0, MODE == kFwdRaw ? ref_mean(L.ref, 1) : 0.0,
+                          MODE == kFwdRaw ? ref_mean(L.ref, 2) : 0.0};
   int t = (int)(w0 / F);
   int64_t f = w0 - (int64_t)t * F;
   for (int64_t w = w0; w < w1; ++w) {
@@ -546,9 +551,9 @@ __global__ void __launch_bounds__(kGatherThreads) rmsd_gather_kernel(const Frame
         const double x0 = x[j][0], x1 = x[j][1], x2 = x[j][2];
         if (MODE == kFwdRaw) {
           if (c0 + lane + 32 * j < a1) {
-            const double d0 = x0 - (y[j][0] + L.ref.mean[0]);
-            const double d1 = x1 - (y[j][1] + L.ref.mean[1]);
-            const double d2 = x2 - (y[j][2] + L.ref.mean[2]);
+            const double d0 = x0 - (y[j][0] + mean[0]);
+            const double d1 = x1 - (y[j][1] + mean[1]);
+            const double d2 = x2 - (y[j][2] + mean[2]);
             acc[0] = fma(d0, d0, acc[0]);
             acc[1] = fma(d1, d1, acc[1]);
             acc[2] = fma(d2, d2, acc[2]);

@@ -106,7 +106,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 // Packed xyz: 4 atoms = 3 swizzled 16-byte chunks; xyzw: 1 atom = 1 chunk.
 template <int STRIDE, bool RAW, bool W>
 __device__ __forceinline__ void stage_sums(double (&acc)[15], const unsigned char* st, int lane, int valid,
-                                           const FrameLaunch& L) {
+                                           const double (&mean)[3]) {
   const float* wb = reinterpret_cast<const float*>(st + LaneGeo<STRIDE>::kXBytes + LaneGeo<STRIDE>::kYBytes);
   const unsigned char* row = st + lane * 128;
   const int sw = lane & 7;
@@ -119,9 +119,9 @@ __device__ __forceinline__ void stage_sums(double (&acc)[15], const unsigned cha
     const double x0 = fx, x1 = fy, x2 = fz;
     if (W && RAW) in = in && wb[k] != 0.0f;  // expanded selection: unselected atoms have weight 0
     if (RAW) {
-      const double d0 = x0 - (y0 + L.ref.mean[0]);
-      const double d1 = x1 - (y1 + L.ref.mean[1]);
-      const double d2 = x2 - (y2 + L.ref.mean[2]);
+      const double d0 = x0 - (y0 + mean[0]);
+      const double d1 = x1 - (y1 + mean[1]);
+      const double d2 = x2 - (y2 + mean[2]);
       acc[0] = fma(d0, in ? d0 : 0.0, acc[0]);
       acc[1] = fma(d1, in ? d1 : 0.0, acc[1]);
       acc[2] = fma(d2, in ? d2 : 0.0, acc[2]);
@@ -168,7 +168,7 @@ __device__ __forceinline__ void stage_sums(double (&acc)[15], const unsigned cha
 // row i, from float offset off; atoms at or past `valid` are masked.
 template <bool RAW, bool W>
 __device__ __forceinline__ void stage_sums_quad(double (&acc)[15], const unsigned char* st, int lane, int off,
-                                                int valid, const FrameLaunch& L) {
+                                                int valid, const double (&mean)[3]) {
   const float* wb = reinterpret_cast<const float*>(st + QuadGeo::kXBytes + QuadGeo::kYBytes);
   const float* row =
       reinterpret_cast<const float*>(st + (lane & 3) * QuadGeo::kBoxBytes + (lane >> 2) * QuadGeo::kBoxRowBytes) + off;
@@ -180,9 +180,9 @@ __device__ __forceinline__ void stage_sums_quad(double (&acc)[15], const unsigne
     const double y0 = yb[3 * k], y1 = yb[3 * k + 1], y2 = yb[3 * k + 2];
     if (RAW) {
       const bool in = !W || wb[k] != 0.0f;
-      const double d0 = x0 - (y0 + L.ref.mean[0]);
-      const double d1 = x1 - (y1 + L.ref.mean[1]);
-      const double d2 = x2 - (y2 + L.ref.mean[2]);
+      const double d0 = x0 - (y0 + mean[0]);
+      const double d1 = x1 - (y1 + mean[1]);
+      const double d2 = x2 - (y2 + mean[2]);
       acc[0] = fma(d0, in ? d0 : 0.0, acc[0]);
       acc[1] = fma(d1, in ? d1 : 0.0, acc[1]);
       acc[2] = fma(d2, in ? d2 : 0.0, acc[2]);
@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
   // quad rows: this lane's float offset into its box row (stages start at
   // multiples of 32 atoms, so only the frame position matters)
   const int quad_off = QUAD ? (int)(((int64_t)(lane & 3) * 3 * L.n_atoms) & 3) : 0;
+  const double mean[3] = {RAW ? ref_mean(L.ref, 0) : 0.0, RAW ? ref_mean(L.ref, 1) : 0.0, RAW ? ref_mean(L.ref, 2) : 0.0};
   int64_t n_done = 0;
   bool aborted = false;
   for (int64_t u = u0; u < u1 && !aborted; ++u) {
@@ -297,9 +298,9 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
       const int64_t a0 = t * tile + (int64_t)k * kLaneAtoms;
       const int valid = (int)min((int64_t)kLaneAtoms, n_sel - a0);
       if (QUAD)
-        stage_sums_quad<RAW, W>(acc, ring + slot * G::kStageBytes, lane, quad_off, valid, L);
+        stage_sums_quad<RAW, W>(acc, ring + slot * G::kStageBytes, lane, quad_off, valid, mean);
       else
-        stage_sums<STRIDE, RAW, W>(acc, ring + slot * G::kStageBytes, lane, valid, L);
+        stage_sums<STRIDE, RAW, W>(acc, ring + slot * G::kStageBytes, lane, valid, mean);
       ++n_done;
       __syncwarp();
       if (lane == 0 && pu < u1) issue_next();

@@ -71,8 +71,7 @@ struct VgArgs {
   int G = 32;                  // frames per group (TMA box rows)
   int64_t n_groups = 0;
   const double* yc = nullptr;  // [n_atoms + 32][3] centred reference, FP64, zero-padded
-  double sum_c[3] = {0, 0, 0};
-  double gy = 0;
+  RefInfo ref;                 // its scalars
   double* rmsd = nullptr;      // [F] or null
   double* stats = nullptr;     // [F][16]: written by forward, read by backward
   const void* w = nullptr;     // per-frame dL/drmsd, or null (1)
@@ -289,18 +288,19 @@ __global__ void __launch_bounds__(kVgThreads, 1) rmsd_vg_kernel(const __grid_con
 #pragma unroll
           for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) h[a * 3 + b] = t[6 + a * 3 + b] - sx[a] * A.sum_c[b] * inv_n;
+            for (int b = 0; b < 3; ++b) h[a * 3 + b] = t[6 + a * 3 + b] - sx[a] * ref_sum_c(A.ref, b) * inv_n;
           const double gx = t[3] + t[4] + t[5] - (sx[0] * sx[0] + sx[1] * sx[1] + sx[2] * sx[2]) * inv_n;
-          const QcpOut q = qcp_lambda(h, 0.5 * (gx + A.gy));
-          const double rmsd = sqrt(msd_from(gx, A.gy, q.lambda, n));
-          flag = rmsd < kRefineScale * (gx + A.gy) * inv_n;
+          const double gy = ref_gy(A.ref);
+          const QcpOut q = qcp_lambda(h, 0.5 * (gx + gy));
+          const double rmsd = sqrt(msd_from(gx, gy, q.lambda, n));
+          flag = rmsd < kRefineScale * (gx + gy) * inv_n;
           if (A.rmsd) A.rmsd[f] = rmsd;
           if (A.stats) {
             double* st = A.stats + f * kStatDoubles;
             st[0] = sx[0] * inv_n; st[1] = sx[1] * inv_n; st[2] = sx[2] * inv_n;
 #pragma unroll
             for (int e = 0; e < 9; ++e) st[3 + e] = h[e];
-            st[12] = q.lambda; st[13] = rmsd; st[14] = n; st[15] = gx + A.gy;
+            st[12] = q.lambda; st[13] = rmsd; st[14] = n; st[15] = gx + gy;
           }
           c[0] = sx[0] * inv_n; c[1] = sx[1] * inv_n; c[2] = sx[2] * inv_n;
           if (MODE == kVgBoth || flag) rotation_from_qcp(h, q.lambda, R);
@@ -338,7 +338,8 @@ __global__ void __launch_bounds__(kVgThreads, 1) rmsd_vg_kernel(const __grid_con
       for (int e = 0; e < 9; ++e) R[e] = fr[kFrmR + e];
       c[0] = fr[kFrmC]; c[1] = fr[kFrmC + 1]; c[2] = fr[kFrmC + 2];
       const bool flag = fr[kFrmFlag] != 0.0;
-      const double my0 = A.sum_c[0] * inv_n, my1 = A.sum_c[1] * inv_n, my2 = A.sum_c[2] * inv_n;
+      const double my0 = ref_sum_c(A.ref, 0) * inv_n, my1 = ref_sum_c(A.ref, 1) * inv_n,
+                   my2 = ref_sum_c(A.ref, 2) * inv_n;
       double ra = 0.0;
       run_pass(f0, pre, false, [&](unsigned char* st, int64_t s) {
         const double2* yb = reinterpret_cast<const double2*>(st + kVgXBytes);
@@ -539,8 +540,7 @@ cudaError_t launch_vg(int mode, const VgLaunch& V, int sm_count, cudaStream_t s,
   A.G = G;
   A.n_groups = (V.n_frames + G - 1) / G;
   A.yc = V.ref.yc;
-  for (int c = 0; c < 3; ++c) A.sum_c[c] = V.ref.sum_c[c];
-  A.gy = V.ref.gy;
+  A.ref = V.ref;
   A.rmsd = V.rmsd;
   A.stats = V.stats;
   A.w = V.w;

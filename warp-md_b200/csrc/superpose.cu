@@ -58,13 +58,13 @@ __global__ void __launch_bounds__(256) superpose_finalize_kernel(const FrameLaun
   if (W > 0.0 || W < 0.0) {
     const double inv_w = 1.0 / W;
     cx[0] = tot[0] * inv_w; cx[1] = tot[1] * inv_w; cx[2] = tot[2] * inv_w;
-    cy[0] = L.ref.mean[0]; cy[1] = L.ref.mean[1]; cy[2] = L.ref.mean[2];
+    for (int c = 0; c < 3; ++c) cy[c] = ref_mean(L.ref, c);
     if (!norotate) {
       double h[9];
       for (int a = 0; a < 3; ++a)
-        for (int b = 0; b < 3; ++b) h[a * 3 + b] = tot[6 + a * 3 + b] - cx[a] * L.ref.sum_c[b];
+        for (int b = 0; b < 3; ++b) h[a * 3 + b] = tot[6 + a * 3 + b] - cx[a] * ref_sum_c(L.ref, b);
       const double gx = tot[3] + tot[4] + tot[5] - (tot[0] * cx[0] + tot[1] * cx[1] + tot[2] * cx[2]);
-      const QcpOut q = qcp_lambda(h, 0.5 * (gx + L.ref.gy));
+      const QcpOut q = qcp_lambda(h, 0.5 * (gx + ref_gy(L.ref)));
       rotation_from_qcp(h, q.lambda, r);
     }
   }

@@ -75,6 +75,7 @@ struct HostBuf {
 struct wmd_ref {
   double* yc = nullptr;
   float* w = nullptr;  // per-atom weights (weighted references only)
+  bool owned = true;   // yc and w were allocated for it (else: the caller's workspace)
   wmd::RefInfo info;
 };
 
@@ -654,6 +655,41 @@ WMD_EXPORT int wmd_reference_upload(wmd_ctx* ctx, const float* ref, int64_t n_se
   return reference_upload(ctx, ref, n_sel, stride, nullptr, out);
 }
 
+static size_t ref_yc_bytes(int64_t n_sel) { return ((size_t)(n_sel + 32) * 3 * sizeof(double) + 255) & ~size_t(255); }
+
+WMD_EXPORT size_t wmd_reference_workspace(int64_t n_sel) {
+  return n_sel < 0 ? 0 : ref_yc_bytes(n_sel) + wmd::kRefScalars * sizeof(double);
+}
+
+WMD_EXPORT int wmd_reference_prepare(wmd_ctx* ctx, const float* ref, int64_t n_sel, int stride, void* workspace,
+                                     size_t workspace_bytes, void* stream, wmd_ref** out) {
+  if (!ctx) return WMD_ERR_INVALID_ARG;
+  if (!out) return set_err(ctx, WMD_ERR_INVALID_ARG, "out is null");
+  *out = nullptr;
+  if (stride != 3 && stride != 4) return set_err(ctx, WMD_ERR_INVALID_ARG, "stride must be 3 or 4 (got %d)", stride);
+  if (n_sel < 0) return set_err(ctx, WMD_ERR_INVALID_ARG, "negative size");
+  if (n_sel > 0 && !ref) return set_err(ctx, WMD_ERR_INVALID_ARG, "reference is null");
+  if (!workspace || workspace_bytes < wmd_reference_workspace(n_sel) ||
+      (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
+    return set_err(ctx, WMD_ERR_INVALID_ARG, "the workspace must be 256-byte aligned and hold %zu bytes",
+                   wmd_reference_workspace(n_sel));
+  DeviceGuard g(ctx->device);
+  if ((n_sel > 0 && classify(ref) != Mem::Device) || classify(workspace) != Mem::Device)
+    return set_err(ctx, WMD_ERR_INVALID_ARG, "reference and workspace must be device memory for this entry point");
+  double* yc = static_cast<double*>(workspace);
+  double* scal = reinterpret_cast<double*>(static_cast<char*>(workspace) + ref_yc_bytes(n_sel));
+  CU(wmd::launch_ref_prep(ref, n_sel, stride, yc, scal, static_cast<cudaStream_t>(stream)), "reference");
+  wmd_ref* r = new wmd_ref();
+  r->owned = false;
+  r->yc = yc;
+  r->info.n_sel = n_sel;
+  r->info.wsum = (double)n_sel;
+  r->info.yc = yc;
+  r->info.scal = scal;
+  *out = r;
+  return WMD_OK;
+}
+
 WMD_EXPORT int wmd_reference_upload_weighted(wmd_ctx* ctx, const float* ref, int64_t n_sel, int stride,
                                              const float* weights, wmd_ref** out) {
   return reference_upload(ctx, ref, n_sel, stride, weights, out);
@@ -661,6 +697,10 @@ WMD_EXPORT int wmd_reference_upload_weighted(wmd_ctx* ctx, const float* ref, int
 
 WMD_EXPORT int wmd_reference_free(wmd_ctx* ctx, wmd_ref* ref) {
   if (!ref) return WMD_OK;
+  if (!ref->owned) {
+    delete ref;
+    return WMD_OK;
+  }
   if (ctx) {
     DeviceGuard g(ctx->device);
     cudaFree(ref->yc);

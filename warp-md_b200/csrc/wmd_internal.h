@@ -35,7 +35,19 @@ struct RefInfo {
   double mean[3] = {0, 0, 0};   // mean(y), for the no-fit RMSD
   double sumsq = 0;             // sum |y|^2, for the no-fit RMSD
   double wsum = 0;              // sum of the weights (n_sel when unweighted)
+  // device [kRefScalars], or null: the scalars above as ref_prep_kernel wrote
+  // them (a reference prepared on the device); the members are then unset
+  const double* scal = nullptr;
 };
+enum RefScalar : int { kRefMean = 0, kRefSumC = 3, kRefGy = 6, kRefScalars = 8 };
+#if defined(__CUDACC__)
+__device__ __forceinline__ double ref_mean(const RefInfo& r, int c) { return r.scal ? __ldg(r.scal + kRefMean + c) : r.mean[c]; }
+__device__ __forceinline__ double ref_sum_c(const RefInfo& r, int c) { return r.scal ? __ldg(r.scal + kRefSumC + c) : r.sum_c[c]; }
+__device__ __forceinline__ double ref_gy(const RefInfo& r) { return r.scal ? __ldg(r.scal + kRefGy) : r.gy; }
+#endif
+// Centres a device-resident reference (reference.cu): yc [n_sel + 32][3]
+// (zero-padded) and scal [kRefScalars], all on `s`.
+cudaError_t launch_ref_prep(const float* ref, int64_t n_sel, int stride, double* yc, double* scal, cudaStream_t s);
 
 struct FrameLaunch {
   const float* coords = nullptr;  // device, frames of this launch

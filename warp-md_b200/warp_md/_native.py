@@ -39,7 +39,7 @@ FRAME_STATS = 16
 
 # every symbol include/warpmd_rmsd.h declares
 EXPORTED = (
-    "wmd_create", "wmd_destroy", "wmd_last_error", "wmd_version", "wmd_reference_upload", "wmd_reference_free",
+    "wmd_create", "wmd_destroy", "wmd_last_error", "wmd_version", "wmd_reference_upload", "wmd_reference_free", "wmd_reference_workspace", "wmd_reference_prepare",
     "wmd_rmsd_frames", "wmd_rmsd_forward", "wmd_rmsd_backward", "wmd_rmsd_covariance", "wmd_pairwise_rmsd", "wmd_pairwise_dme",
     "wmd_batched_prepare", "wmd_batched_rmsd", "wmd_batched_layout", "wmd_rmsd_frames_noalloc", "wmd_set_wait_test",
     "wmd_pairwise_rmsd_part", "wmd_rmsd_backward_f64", "wmd_rmsd_value_and_grad",
@@ -92,6 +92,8 @@ def load() -> ctypes.CDLL:
         L.wmd_version.restype = ctypes.c_char_p
         L.wmd_reference_upload.argtypes = [vp, vp, i64, i32, ctypes.POINTER(vp)]
         L.wmd_reference_free.argtypes = [vp, vp]
+        L.wmd_reference_workspace.argtypes = [i64]
+        L.wmd_reference_prepare.argtypes = [vp, vp, i64, i32, vp, ctypes.c_size_t, vp, ctypes.POINTER(vp)]
         L.wmd_set_wait_test.argtypes = [vp, ctypes.c_uint64, i32]
         L.wmd_rmsd_frames.argtypes = [vp, vp, i64, i64, i32, vp, i64, vp, i32, vp, vp]
         L.wmd_rmsd_forward.argtypes = [vp, vp, i64, i64, i32, vp, i64, vp, vp, vp, vp]
@@ -124,6 +126,7 @@ def load() -> ctypes.CDLL:
         L.wmd_dcd_rmsd.argtypes = [vp, vp, i64, i64, vp, i64, vp, i32, vp, ctypes.POINTER(i64), vp]
         for name in EXPORTED:
             getattr(L, name).restype = getattr(L, name).restype if name in ("wmd_last_error", "wmd_version") else i32
+        L.wmd_reference_workspace.restype = ctypes.c_size_t
         _lib = L
         return _lib
 
@@ -186,6 +189,21 @@ class Reference:
         if w.shape != (r.shape[0],):
             raise WarpMdError(WMD_ERR_MISMATCH, "weights must have one entry per reference atom")
         return cls(ctx, r.ctypes.data, r.shape[0], r.shape[1], keepalive=(r, w), weights_ptr=w.ctypes.data)
+
+    @classmethod
+    def prepared(cls, ctx: Context, coords_ptr: int, n_sel: int, stride: int, workspace_ptr: int, workspace_bytes: int,
+                 stream: int, keepalive) -> "Reference":
+        """A reference in device memory, centred on ``stream`` into the
+        caller's workspace (kept alive with the coordinates by ``keepalive``)."""
+        r = cls.__new__(cls)
+        r.ctx = ctx
+        r.n_sel = int(n_sel)
+        r._keep = keepalive
+        h = ctypes.c_void_p()
+        ctx.check(ctx.lib.wmd_reference_prepare(ctx.handle, coords_ptr, int(n_sel), int(stride), workspace_ptr,
+                                                int(workspace_bytes), stream, ctypes.byref(h)))
+        r.handle = h
+        return r
 
     def close(self) -> None:
         if getattr(self, "handle", None) and self.ctx.handle:

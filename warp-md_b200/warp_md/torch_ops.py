@@ -21,20 +21,56 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+class _RefEntry:
+    """A reference centred on one stream, and what calls on others need."""
+
+    def __init__(self, ctx: N.Context, ref: torch.Tensor):
+        self.stream = torch.cuda.current_stream(ref.device)
+        y = ref.detach().to(torch.float32).contiguous()
+        if y.dim() != 2:
+            raise N.WarpMdError(N.WMD_ERR_INVALID_ARG, "reference must have shape (atoms, 3) or (atoms, 4)")
+        size = ctx.lib.wmd_reference_workspace(y.shape[0])
+        self.work = torch.empty(size, dtype=torch.uint8, device=y.device)
+        self.ref = N.Reference.prepared(ctx, y.data_ptr() or None, y.shape[0], y.shape[1], self.work.data_ptr(), size,
+                                        self.stream.cuda_stream, keepalive=(y, self.work))
+        self.done: Optional[torch.cuda.Event] = None  # None: finished
+
+    def usable(self, stream: torch.cuda.Stream, capturing: bool) -> bool:
+        """Orders ``stream`` after the centring kernel.  False while a graph is
+        captured and that kernel is not known to have finished: a capture
+        cannot wait for work outside it."""
+        if self.done is not None and not capturing and self.done.query():
+            self.done = None
+        if capturing:
+            return self.done is None
+        if stream != self.stream:
+            if self.done is not None:
+                stream.wait_event(self.done)
+            self.work.record_stream(stream)
+        return True
+
+
 class _RefCache:
-    """Keeps uploaded references alive per (device, data_ptr, version)."""
+    """Keeps the last centred reference per (device, data_ptr, version, layout);
+    its tensor is kept alive with it, so the address stays its own."""
 
     def __init__(self):
-        self._key = None
-        self._ref = None
+        self._last = (None, None)
 
     def get(self, ctx: N.Context, ref: torch.Tensor) -> N.Reference:
-        key = (ctx.device, ref.data_ptr(), ref._version, tuple(ref.shape))
-        if key != self._key:
-            r = ref.detach().to(torch.float32).contiguous()
-            self._ref = N.Reference(ctx, r.data_ptr(), r.shape[0], r.shape[1], keepalive=r)
-            self._key = key
-        return self._ref
+        key = (ctx.device, ref.data_ptr(), ref._version, tuple(ref.shape), ref.stride(), ref.dtype)
+        with torch.cuda.device(ref.device):
+            stream = torch.cuda.current_stream()
+            capturing = torch.cuda.is_current_stream_capturing()
+            last_key, entry = self._last
+            if key == last_key and entry.usable(stream, capturing):
+                return entry.ref
+            entry = _RefEntry(ctx, ref)
+            if not capturing:  # a captured centring runs only when the graph does
+                entry.done = torch.cuda.Event()
+                entry.done.record(stream)
+                self._last = (key, entry)
+            return entry.ref
 
 
 _cache = _RefCache()
