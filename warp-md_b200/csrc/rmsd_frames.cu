@@ -39,12 +39,11 @@
 #include <cstdint>
 
 #include "device_util.cuh"
+#include "frame_parts.cuh"
 #include "qcp.cuh"
 #include "wmd_internal.h"
 
 namespace wmd {
-
-enum Mode : int { kFwdFit = 0, kFwdRaw = 1, kBwd = 2, kFwdW = 3 };
 
 template <int STRIDE, int APT>
 struct Geo {
@@ -61,57 +60,6 @@ struct Geo {
   static constexpr int kSmemBytes = kAbortOffset + 16;
 };
 
-// Everything a finished frame needs: the 15 CTA/partial sums in lanes 0..14.
-__device__ __noinline__ void finish_frame(const FrameLaunch& L, int64_t f, double v, int mode) {
-  double tot[16];
-#pragma unroll
-  for (int e = 0; e < 16; ++e) tot[e] = __shfl_sync(0xffffffffu, v, e);
-  if ((threadIdx.x & 31) != 0) return;
-  const double n = (double)L.ref.n_sel;
-  if (mode == kFwdRaw) {
-    // tot[0] = sum |x - y|^2 accumulated directly
-    const double msd = n > 0 ? tot[0] / n : 0.0;
-    if (L.out.rmsd) L.out.rmsd[f] = sqrt(msd);
-    return;
-  }
-  const double inv_n = 1.0 / n;
-  const double sx[3] = {tot[0], tot[1], tot[2]};
-  const double sxx = tot[3] + tot[4] + tot[5];
-  double h[9];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) h[a * 3 + b] = tot[6 + a * 3 + b] - sx[a] * ref_sum_c(L.ref, b) * inv_n;
-  const double gx = sxx - (sx[0] * sx[0] + sx[1] * sx[1] + sx[2] * sx[2]) * inv_n;
-  const double gy = ref_gy(L.ref);
-  const QcpOut q = qcp_lambda(h, 0.5 * (gx + gy));
-  const double rmsd = sqrt(msd_from(gx, gy, q.lambda, n));
-  if (L.out.rmsd) L.out.rmsd[f] = rmsd;
-  if (L.refine && (L.out.rmsd || L.out.stats) && rmsd < kRefineScale * (gx + gy) * inv_n) {
-    // near-zero RMSD: queue the frame for the explicit residual pass
-    const unsigned slot = atomicAdd(L.refine_count, 1u);
-    double* rec = L.refine + (size_t)slot * kStatDoubles;
-    rec[0] = (double)f;
-    rec[1] = sx[0] * inv_n; rec[2] = sx[1] * inv_n; rec[3] = sx[2] * inv_n;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) rec[4 + e] = h[e];
-    rec[13] = q.lambda;
-  }
-  if (L.out.stats) {
-    double* st = L.out.stats + f * kStatDoubles;
-    st[0] = sx[0] * inv_n; st[1] = sx[1] * inv_n; st[2] = sx[2] * inv_n;
-#pragma unroll
-    for (int e = 0; e < 9; ++e) st[3 + e] = h[e];
-    st[12] = q.lambda; st[13] = rmsd; st[14] = n; st[15] = gx + gy;
-  }
-  if (L.out.cov) {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) L.out.cov[f * 9 + e] = (float)h[e];
-  }
-  if (L.out.sum_x2) L.out.sum_x2[f] = (float)gx;
-  if (L.out.sum_y2) L.out.sum_y2[f] = (float)gy;
-}
-
 // Leader warp of an item: total over the 8 consumer warps, stored as the
 // item's 16-double partial.  No fence and no atomic here: frames are finished
 // by rmsd_finalize_kernel after the streaming kernel has ended.
@@ -127,18 +75,32 @@ __device__ __forceinline__ void item_epilogue(const FrameLaunch& L, const double
 }
 
 // One warp per frame: adds the frame's tile partials in tile order (so results
-// are bitwise reproducible), then QCP / outputs in finish_frame.
+// are bitwise reproducible), then QCP / outputs in finish_totals.  Bound by the
+// latency of the records: with one in flight per lane pair it took 33 us for
+// 4,000 frames x 196 tiles, with 16 in flight 14.5 us.
 template <int MODE>
 __global__ void __launch_bounds__(256) rmsd_finalize_kernel(const FrameLaunch L, int n_tiles) {
   const int64_t f = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (f >= L.n_frames) return;
   const int lane = threadIdx.x & 31;
+  // lanes 0-15 read the even tiles, lanes 16-31 the odd ones, 16 tiles in flight;
+  // lanes 0-15 add them in tile order
+  const double* part = L.partial + (size_t)f * n_tiles * kStatDoubles + (lane & 15);
   double s = 0.0;
-  if (lane < 16) {
-    const double* part = L.partial + (size_t)f * n_tiles * kStatDoubles + lane;
-    for (int tt = 0; tt < n_tiles; ++tt) s += part[(size_t)tt * kStatDoubles];
+  for (int t0 = lane >> 4; t0 < n_tiles + (lane >> 4); t0 += 16) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = t0 + 2 * u < n_tiles ? part[(size_t)(t0 + 2 * u) * kStatDoubles] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      s += v[u];
+      s += __shfl_down_sync(0xffffffffu, v[u], 16);
+    }
   }
-  finish_frame(L, f, s, MODE);
+  double tot[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) tot[e] = __shfl_sync(0xffffffffu, s, e);
+  if (lane == 0) finish_totals(L, f, tot, MODE);
 }
 
 // Byte range of item (t, f) and its bulk copy into a stage.  The 16-byte
@@ -485,21 +447,7 @@ __global__ void __launch_bounds__(256) rmsd_refine_kernel(const FrameLaunch L) {
 // positions, all of a sub-chunk's loads in flight before any use, and
 // reduces its sums with shuffles.  Latency is hidden by the warps resident
 // per SM instead of by a CTA-wide pipeline.
-//
-// An atom's 12 bytes cost two loads, not three: an 8-byte load of the pair
-// that starts on an 8-byte boundary (x,y or y,z) and a 4-byte load of the
-// other coordinate.
-constexpr int kGatherJ = 4;
 constexpr int kGatherThreads = 128;
-
-__device__ __forceinline__ void load_xyz(const float* p, float& x, float& y, float& z) {
-  const bool odd = (reinterpret_cast<uintptr_t>(p) & 7u) != 0;
-  const float2 pr = __ldg(reinterpret_cast<const float2*>(p + (odd ? 1 : 0)));
-  const float s = __ldg(p + (odd ? 0 : 2));
-  x = odd ? s : pr.x;
-  y = odd ? pr.x : pr.y;
-  z = odd ? pr.y : s;
-}
 
 template <int STRIDE, int MODE>
 __global__ void __launch_bounds__(kGatherThreads) rmsd_gather_kernel(const FrameLaunch L, int tile) {
@@ -519,66 +467,7 @@ __global__ void __launch_bounds__(kGatherThreads) rmsd_gather_kernel(const Frame
     const int64_t a0 = (int64_t)t * tile;
     const int64_t a1 = min(n_sel, a0 + tile);
     const float* frame = L.coords + (size_t)f * L.n_atoms * STRIDE;
-    double acc[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
-#pragma unroll 1
-    for (int64_t c0 = a0; c0 < a1; c0 += 32 * kGatherJ) {
-      float x[kGatherJ][3];
-      double y[kGatherJ][3];
-      float wt[MODE == kFwdW ? kGatherJ : 1];
-#pragma unroll
-      for (int j = 0; j < kGatherJ; ++j) {
-        const int64_t k = c0 + lane + 32 * j;
-        if (k < a1) {
-          int64_t idx = L.sel ? (int64_t)__ldg(L.sel + k) : k;
-          if (idx >= L.n_atoms) {  // bad device-side selection: report, read atom 0
-            atomicOr(L.status, kStatusBadIndex);
-            idx = 0;
-          }
-          load_xyz(frame + idx * STRIDE, x[j][0], x[j][1], x[j][2]);
-          const double* yp = L.ref.yc + k * 3;
-          y[j][0] = __ldg(yp); y[j][1] = __ldg(yp + 1); y[j][2] = __ldg(yp + 2);
-          if (MODE == kFwdW) wt[MODE == kFwdW ? j : 0] = __ldg(L.ref.w + k);
-        } else {
-          x[j][0] = x[j][1] = x[j][2] = 0.f;
-          y[j][0] = y[j][1] = y[j][2] = 0.0;
-          if (MODE == kFwdW) wt[MODE == kFwdW ? j : 0] = 0.f;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kGatherJ; ++j) {
-        const double x0 = x[j][0], x1 = x[j][1], x2 = x[j][2];
-        if (MODE == kFwdRaw) {
-          if (c0 + lane + 32 * j < a1) {
-            const double d0 = x0 - (y[j][0] + mean[0]);
-            const double d1 = x1 - (y[j][1] + mean[1]);
-            const double d2 = x2 - (y[j][2] + mean[2]);
-            acc[0] = fma(d0, d0, acc[0]);
-            acc[1] = fma(d1, d1, acc[1]);
-            acc[2] = fma(d2, d2, acc[2]);
-          }
-        } else {
-          if (MODE == kFwdW) {
-            const double wj = wt[MODE == kFwdW ? j : 0];
-            const double u0 = wj * x0, u1 = wj * x1, u2 = wj * x2;
-            acc[0] += u0; acc[1] += u1; acc[2] += u2;
-            acc[3] = fma(u0, x0, acc[3]); acc[4] = fma(u1, x1, acc[4]); acc[5] = fma(u2, x2, acc[5]);
-          } else {
-            acc[0] += x0; acc[1] += x1; acc[2] += x2;
-            acc[3] = fma(x0, x0, acc[3]); acc[4] = fma(x1, x1, acc[4]); acc[5] = fma(x2, x2, acc[5]);
-          }
-          acc[6] = fma(x0, y[j][0], acc[6]);  acc[7] = fma(x0, y[j][1], acc[7]);  acc[8] = fma(x0, y[j][2], acc[8]);
-          acc[9] = fma(x1, y[j][0], acc[9]);  acc[10] = fma(x1, y[j][1], acc[10]); acc[11] = fma(x1, y[j][2], acc[11]);
-          acc[12] = fma(x2, y[j][0], acc[12]); acc[13] = fma(x2, y[j][1], acc[13]); acc[14] = fma(x2, y[j][2], acc[14]);
-        }
-      }
-    }
-    if (MODE == kFwdRaw) {
-      acc[0] += acc[1] + acc[2];
-      acc[1] = acc[2] = 0.0;
-    }
-    const double v = warp_reduce_scatter16(acc);
+    const double v = gather_item<STRIDE, MODE>(L, frame, a0, a1, mean, lane);
     if ((lane & 1) == 0) L.partial[((size_t)f * n_tiles + t) * kStatDoubles + (lane >> 1)] = v;
     if (++f == F) { f = 0; ++t; }
   }
@@ -694,23 +583,29 @@ int frame_grid(const FrameLaunch& L, int sm_count, bool backward) {
 
 cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s) {
   if (L.n_frames == 0) return cudaSuccess;
-  if (!L.align) {
-    cudaError_t e = L.lanes ? launch_lanes_forward(L, true, s) : dispatch<kFwdRaw>(L, s);
-    if (e != cudaSuccess) return e;
-    rmsd_finalize_kernel<kFwdRaw><<<(unsigned)((L.n_frames + 7) / 8), 256, 0, s>>>(L, frame_tiles(L));
-    return cudaGetLastError();
-  }
-  if (L.refine) {
-    cudaError_t e = cudaMemsetAsync(L.refine_count, 0, sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
-  }
-  cudaError_t e = L.lanes ? launch_lanes_forward(L, false, s) : dispatch<kFwdFit>(L, s);
+  FrameLaunch K = L;
+  // few tiles per frame: the frames-across-lanes kernel finishes its frames itself
+  const bool fused = L.lanes && L.group_done && frame_tiles(L) <= kLaneFinishTiles && L.n_frames >= 4;
+  if (!fused) K.group_done = nullptr;
+  const bool refine = L.align && L.refine;
+  cudaError_t e = cudaSuccess;
+  const size_t done_bytes = fused ? (size_t)frame_groups(L.n_frames) * sizeof(unsigned) : 0;
+  if (refine) e = cudaMemsetAsync(L.refine_count, 0, sizeof(unsigned) + done_bytes, s);
+  else if (fused) e = cudaMemsetAsync(L.group_done, 0, done_bytes, s);
   if (e != cudaSuccess) return e;
-  rmsd_finalize_kernel<kFwdFit><<<(unsigned)((L.n_frames + 7) / 8), 256, 0, s>>>(L, frame_tiles(L));
-  if ((e = cudaGetLastError()) != cudaSuccess || !L.refine) return e;
+  if (L.align) e = L.lanes ? launch_lanes_forward(K, false, s) : dispatch<kFwdFit>(K, s);
+  else e = L.lanes ? launch_lanes_forward(K, true, s) : dispatch<kFwdRaw>(K, s);
+  if (e != cudaSuccess) return e;
+  if (!fused) {
+    const unsigned blocks = (unsigned)((L.n_frames + 7) / 8);
+    if (L.align) rmsd_finalize_kernel<kFwdFit><<<blocks, 256, 0, s>>>(K, frame_tiles(L));
+    else rmsd_finalize_kernel<kFwdRaw><<<blocks, 256, 0, s>>>(K, frame_tiles(L));
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (!refine) return cudaSuccess;
   const int blocks = (int)std::min<int64_t>(L.n_frames, 148);
-  if (L.stride == 4) rmsd_refine_kernel<4><<<blocks, 256, 0, s>>>(L);
-  else rmsd_refine_kernel<3><<<blocks, 256, 0, s>>>(L);
+  if (L.stride == 4) rmsd_refine_kernel<4><<<blocks, 256, 0, s>>>(K);
+  else rmsd_refine_kernel<3><<<blocks, 256, 0, s>>>(K);
   return cudaGetLastError();
 }
 

@@ -13,7 +13,7 @@
 //     by lane 0 as soon as the warp is done with one.
 //   * Each lane adds, in FP64 and in atom order, the 15 sums of its own frame
 //     (sum x, sum x_a^2, sum x y_c^T): no shuffles, no barriers.
-//   * Atoms are grouped into tiles (256 to 2,048 atoms, chosen per launch so
+//   * Atoms are grouped into tiles (128 to 2,048 atoms, chosen per launch so
 //     that whole units balance over the warp slots); a unit is (tile,
 //     32-frame group) and belongs to one warp, which stores each lane's 16 sums into
 //     the same [frame][tile][16] partials the finalize kernel reads.  Every
@@ -29,8 +29,18 @@
 // floats at a fixed offset of (3 j n_atoms) mod 4 floats with 32-bit loads:
 // rows of 400 bytes put the 32 lanes in distinct banks for odd n_atoms (two
 // lanes per bank otherwise).  Atoms past the tile come from the next frame of
-// the quad row and are masked.  The last n_frames mod 4 frames are left to the
-// gathered kernel, with the same tiles and partial layout.
+// the quad row and are masked.  The last n_frames mod 4 frames are no quad row:
+// their tiles are summed with plain loads, atoms across lanes, by the last warps
+// of the grid (those without units of their own, where there are any) before
+// their units.  As a launch behind this kernel they cost 12 us of 83 for 5,001
+// frames x 3,001 atoms.
+//
+// Finishing.  With L.group_done set, the warp that stores a frame group's last
+// tile adds the group's tiles in tile order and runs QCP, one frame per lane,
+// while other warps still stream: the separate finalize kernel (a warp per frame,
+// QCP on one lane) took 16 us of those 83.  Up to kLaneFinishTiles tiles: a lane
+// reads its frame's records one after another, so with hundreds of them the
+// finalize kernel, a warp per frame, is ahead.
 //
 // Atoms streamed: a dense selection (the first n_sel atoms), or the span
 // [lane_atom0, lane_atom0 + lane_atoms) of a sorted selection with the
@@ -50,6 +60,7 @@
 #include <cstring>
 
 #include "device_util.cuh"
+#include "frame_parts.cuh"
 #include "wmd_internal.h"
 
 namespace wmd {
@@ -224,6 +235,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
   const int64_t units = groups * n_tiles;  // (tile, frame group), tile-major
   const int64_t nw = L.lane_warps, gw = (int64_t)blockIdx.x * kLaneWarps + warp;
   const int64_t u0 = units * gw / nw, u1 = units * (gw + 1) / nw;
+  constexpr int kMode = RAW ? kFwdRaw : kFwdFit;
+  const double mean[3] = {RAW ? ref_mean(L.ref, 0) : 0.0, RAW ? ref_mean(L.ref, 1) : 0.0, RAW ? ref_mean(L.ref, 2) : 0.0};
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kLaneWarps * kLaneStages; ++i) mbar_init(&bars[i], 1);
@@ -231,6 +244,48 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
     fence_barrier_init();
   }
   __syncthreads();
+
+  // this warp has stored its records of group g's tile (lane: frame f, if any):
+  // true when they were the last of the group's
+  auto last_of_group = [&](int64_t g) {
+    __threadfence();
+    __syncwarp();
+    unsigned before = 0;
+    if (lane == 0) before = atomicAdd(L.group_done + g, 1u);
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (before + 1u != (unsigned)n_tiles) return false;
+    __threadfence();
+    return true;
+  };
+  auto finish_from_records = [&](int64_t f) {
+    const double2* rec = reinterpret_cast<const double2*>(L.partial + (size_t)f * n_tiles * kStatDoubles);
+    double tot[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) tot[e] = 0.0;
+#pragma unroll 2
+    for (int t = 0; t < n_tiles; ++t)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const double2 v = __ldcg(rec + t * 8 + e);
+        tot[2 * e] += v.x;
+        tot[2 * e + 1] += v.y;
+      }
+    finish_totals(L, f, tot, kMode);
+  };
+
+  if (QUAD && L.tail_frames > 0) {
+    const int64_t warps = (int64_t)gridDim.x * kLaneWarps;
+    for (int64_t t = warps - 1 - gw; t < n_tiles; t += warps) {
+      for (int64_t f = F; f < F + L.tail_frames; ++f) {
+        const int64_t a0 = t * tile, a1 = min(n_sel, a0 + tile);
+        const double v = gather_item<3, RAW ? kFwdRaw : (W ? kFwdW : kFwdFit)>(L, L.coords + (size_t)f * L.n_atoms * 3, a0,
+                                                                             a1, mean, lane);
+        if ((lane & 1) == 0) L.partial[((size_t)f * n_tiles + t) * kStatDoubles + (lane >> 1)] = v;
+      }
+      if (L.group_done && last_of_group(groups) && lane < L.tail_frames) finish_from_records(F + lane);
+      __syncwarp();
+    }
+  }
   if (gw >= nw || u0 >= u1) return;
 
   auto unit_stages = [&](int64_t u) {
@@ -279,7 +334,6 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
   // quad rows: this lane's float offset into its box row (stages start at
   // multiples of 32 atoms, so only the frame position matters)
   const int quad_off = QUAD ? (int)(((int64_t)(lane & 3) * 3 * L.n_atoms) & 3) : 0;
-  const double mean[3] = {RAW ? ref_mean(L.ref, 0) : 0.0, RAW ? ref_mean(L.ref, 1) : 0.0, RAW ? ref_mean(L.ref, 2) : 0.0};
   int64_t n_done = 0;
   bool aborted = false;
   for (int64_t u = u0; u < u1 && !aborted; ++u) {
@@ -311,11 +365,26 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
       acc[1] = acc[2] = 0.0;
     }
     const int64_t f = g * 32 + lane;
+    if (L.group_done && n_tiles == 1) {  // the unit is the frame
+      if (f < F) {
+        double tot[16];
+#pragma unroll
+        for (int e = 0; e < 15; ++e) tot[e] = acc[e];
+        tot[15] = 0.0;
+        finish_totals(L, f, tot, kMode);
+      }
+      __syncwarp();
+      continue;
+    }
     if (f < F) {
       double2* rec = reinterpret_cast<double2*>(L.partial + ((size_t)f * n_tiles + t) * kStatDoubles);
 #pragma unroll
       for (int e = 0; e < 7; ++e) rec[e] = make_double2(acc[2 * e], acc[2 * e + 1]);
       rec[7] = make_double2(acc[14], 0.0);
+    }
+    if (L.group_done) {
+      if (last_of_group(g) && f < F) finish_from_records(f);
+      __syncwarp();
     }
   }
 
@@ -476,13 +545,14 @@ bool lanes_worthwhile(const FrameLaunch& L, int sm_count) {
 }
 
 int lanes_tile(const FrameLaunch& L, int sm_count) {
-  // Tile size from 2,048 down to 256 atoms minimising the busiest warp's
-  // bytes: (units per warp) x (tile bytes + its 128-byte partial, written
-  // and read back).  Large tiles mean few records; small ones balance short
-  // runs (few frames or few atoms) over all warp slots.
+  // Tile size, any multiple of 32 from 128 to 2,048 atoms, minimising the
+  // busiest warp's bytes: (units per warp) x (tile bytes + its 128-byte partial,
+  // written and read back).  Large tiles mean few records; small ones balance
+  // short runs (few frames or few atoms) over all warp slots.  5,001 frames x
+  // 3,001 atoms: 448 atoms (1,099 units on 1,184 slots) instead of 512 (942).
   const int64_t slots = lanes_slots(L, sm_count);
   int64_t best = kLaneTile, best_cost = -1;
-  for (int64_t tile = kLaneTile; tile >= 256; tile /= 2) {
+  for (int64_t tile = kLaneTile; tile >= 128; tile -= kLaneAtoms) {
     const int64_t per = (lane_units(L, tile) + slots - 1) / slots;
     const int64_t cost = per * (tile * L.stride * 4 + 256);
     if (best_cost < 0 || cost < best_cost) {
@@ -501,26 +571,22 @@ cudaError_t launch_lanes_forward(const FrameLaunch& L, bool raw, cudaStream_t s)
   FrameLaunch K = L;
   const bool w = L.lane_w != nullptr;
   if (lanes_quad(L)) {
-    // whole quad rows here; the last n_frames mod 4 frames by the gathered
-    // kernel into the same partial layout
+    // whole quad rows, and the last n_frames mod 4 frames with plain loads
     const int64_t main = L.n_frames & ~int64_t(3);
     if (main > 0) {  // a batch of fewer than 4 frames has no quad row
       K.n_frames = main;
+      K.tail_frames = (int)(L.n_frames - main);
       K.lane_warps = (int)lane_warps(K, (int64_t)L.grid * kLaneWarps);
       cudaError_t e = w ? (raw ? launch_lanes<3, true, true, true>(K, s) : launch_lanes<3, false, true, true>(K, s))
                         : (raw ? launch_lanes<3, true, false, true>(K, s) : launch_lanes<3, false, false, true>(K, s));
-      if (e != cudaSuccess || main == L.n_frames) return e;
+      return e;
     }
-    FrameLaunch T = L;
-    T.coords = L.coords + (size_t)main * L.n_atoms * 3;
-    T.n_frames = L.n_frames - main;
-    T.partial = L.partial + (size_t)main * frame_tiles(L) * kStatDoubles;
     static int sms[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    return launch_gather_partials(T, raw, sms[dev], s);
+    return launch_gather_partials(L, raw, sms[dev], s);
   }
   K.lane_warps = (int)lane_warps(L, (int64_t)L.grid * kLaneWarps);
   if (L.stride == 4) {

@@ -385,16 +385,18 @@ int forward_device(wmd_ctx* ctx, const float* dcoords, int64_t n_frames, int64_t
   if (align) {
     int rc = ensure(ctx, ctx->refine, (size_t)batch * wmd::kStatDoubles * sizeof(double));
     if (rc) return rc;
-    rc = ensure(ctx, ctx->refine_count, sizeof(unsigned), true);
-    if (rc) return rc;
   }
+  // the refine count and the frame groups' tile counts
+  if (int rc = ensure(ctx, ctx->refine_count, (size_t)(1 + wmd::frame_groups(batch)) * sizeof(unsigned), true)) return rc;
+  unsigned* counts = static_cast<unsigned*>(ctx->refine_count.ptr);
   for (int64_t f0 = 0; f0 < n_frames; f0 += batch) {
     const int64_t nf = std::min(batch, n_frames - f0);
     wmd::FrameLaunch B = L;
     if (align) {
       B.refine = static_cast<double*>(ctx->refine.ptr);
-      B.refine_count = static_cast<unsigned*>(ctx->refine_count.ptr);
+      B.refine_count = counts;
     }
+    B.group_done = counts + 1;
     B.coords = dcoords + (size_t)f0 * n_atoms * stride;
     keep_aligned(B);
     B.n_frames = nf;

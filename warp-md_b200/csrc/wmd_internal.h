@@ -59,6 +59,7 @@ struct FrameLaunch {
   int tile_atoms = 2048;          // atoms per tile (kConsumerThreads * atoms/thread, or kLaneTile)
   bool lanes = false;             // frames-across-lanes forward kernel (rmsd_lanes.cu)
   int lane_warps = 0;             // its active warps (set at launch)
+  int tail_frames = 0;            // its frames past n_frames that fill no quad row (set at launch)
   int64_t lane_atom0 = 0;         // its atoms: [lane_atom0, lane_atom0 + lane_atoms) of every frame
   int64_t lane_atoms = 0;
   const double* lane_y = nullptr; // reference values over those atoms (centred, weighted), +32 zero atoms
@@ -73,6 +74,8 @@ struct FrameLaunch {
   double* partial = nullptr;    // [n_frames][n_tiles][16] per-tile sums
   double* refine = nullptr;     // [n_frames][16] records of frames needing the residual pass
   unsigned* refine_count = nullptr;  // number of records, zeroed before each forward
+  unsigned* group_done = nullptr;    // [frame_groups] tiles stored per 32-frame group, follows *refine_count
+                                     // (cleared with it), or null: rmsd_finalize_kernel finishes the frames
   int* status = nullptr;        // device-visible status word (mapped host)
   WaitCfg wait;                 // limits of the bounded waits
   int grid = 0;                 // CTAs (persistent)
@@ -104,6 +107,10 @@ cudaError_t launch_lanes_forward(const FrameLaunch& L, bool raw, cudaStream_t s)
 cudaError_t launch_lanes_expand(const uint32_t* sel, int64_t n_sel, int64_t a0, const double* yc, const float* w,
                                 double* y_exp, float* w_exp, cudaStream_t s);
 size_t frame_smem_bytes(int stride, int tile_atoms);
+// Entries of FrameLaunch::group_done: the 32-frame groups and the tail.
+inline int64_t frame_groups(int64_t n_frames) { return (n_frames + 31) / 32 + 1; }
+// Most tiles a lane adds up itself (rmsd_lanes.cu)
+constexpr int kLaneFinishTiles = 16;
 // Forward: zeroes L.refine_count, runs the fused kernel, then the residual pass
 // over the frames it flagged.
 cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s);
