@@ -59,6 +59,28 @@ __device__ __forceinline__ void finish_totals(const FrameLaunch& L, int64_t f, c
   if (L.out.sum_y2) L.out.sum_y2[f] = (float)gy;
 }
 
+// A frame's superposition onto the reference from its (weighted) sums: r starts as
+// the identity and stays so with norotate or zero total weight; t = c_y - R c_x.
+__device__ __forceinline__ void transform_from_totals(const RefInfo& ref, const double* tot, int norotate,
+                                                      double (&r)[9], double (&t)[3]) {
+  const double W = ref.wsum;
+  double cx[3] = {0, 0, 0}, cy[3] = {0, 0, 0};
+  if (W > 0.0 || W < 0.0) {
+    const double inv_w = 1.0 / W;
+    cx[0] = tot[0] * inv_w; cx[1] = tot[1] * inv_w; cx[2] = tot[2] * inv_w;
+    for (int c = 0; c < 3; ++c) cy[c] = ref_mean(ref, c);
+    if (!norotate) {
+      double h[9];
+      for (int a = 0; a < 3; ++a)
+        for (int b = 0; b < 3; ++b) h[a * 3 + b] = tot[6 + a * 3 + b] - cx[a] * ref_sum_c(ref, b);
+      const double gx = tot[3] + tot[4] + tot[5] - (tot[0] * cx[0] + tot[1] * cx[1] + tot[2] * cx[2]);
+      const QcpOut q = qcp_lambda(h, 0.5 * (gx + ref_gy(ref)));
+      rotation_from_qcp(h, q.lambda, r);
+    }
+  }
+  for (int i = 0; i < 3; ++i) t[i] = cy[i] - (r[i * 3 + 0] * cx[0] + r[i * 3 + 1] * cx[1] + r[i * 3 + 2] * cx[2]);
+}
+
 // Positions per lane whose loads are in flight together in gather_item.
 constexpr int kGatherJ = 4;
 

@@ -10,7 +10,7 @@
 //   1. the per-frame statistics stream through rmsd_frames_kernel (weighted
 //      mode when the reference carries weights) into tile partials;
 //   2. superpose_finalize_kernel sums each frame's partials in tile order and
-//      runs, one lane per frame, QCP and the rotation from the QCP
+//      runs, a lane per frame, QCP and the rotation from the QCP
 //      eigenvector in FP64 (the same rotation the SVD gives, with the
 //      reflection handled by construction), writing the 12-number transform;
 //   3. superpose_apply_staged (packed, aligned buffers) or
@@ -22,6 +22,7 @@
 #include <cstdint>
 
 #include "device_util.cuh"
+#include "frame_parts.cuh"
 #include "qcp.cuh"
 #include "superpose.h"
 #include "wmd_internal.h"
@@ -29,48 +30,39 @@
 namespace wmd {
 namespace {
 
-// One lane per frame.  xf64[f*16 + 0..8] = R (row-major, R (x - c_x) ~ y - c_y),
-// [9..11] = t; xf32[f*12 + ...] the same rounded to float32 (optional).
-__global__ void __launch_bounds__(256) superpose_finalize_kernel(const FrameLaunch L, int n_tiles, int norotate,
-                                                                 double* __restrict__ xf64,
-                                                                 float* __restrict__ xf32) {
-  __shared__ double st[8][32][17];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t base = ((int64_t)blockIdx.x * 8 + warp) * 32;
-  if (base >= L.n_frames) return;
-  for (int i = 0; i < 16; ++i) {
+// xf64[f*16 + 0..8] = R (row-major, R (x - c_x) ~ y - c_y), [9..11] = t;
+// xf32[f*12 + ...] the same rounded to float32 (optional).  A warp takes
+// kFinFrames frames: it adds their tile partials in tile order, two frames at a
+// time (16 lanes each, 8 records in flight), then runs QCP on a lane per frame.
+// Bound by latency: with 32 frames per warp a thousand frames left all but four
+// SMs idle (1,000 frames x 10 tiles: 30 -> 10 us).
+constexpr int kFinFrames = 8;
+
+__global__ void __launch_bounds__(32) superpose_finalize_kernel(const FrameLaunch L, int n_tiles, int norotate,
+                                                                double* __restrict__ xf64, float* __restrict__ xf32) {
+  __shared__ double st[kFinFrames][17];
+  const int lane = threadIdx.x;
+  const int64_t base = (int64_t)blockIdx.x * kFinFrames;
+#pragma unroll
+  for (int i = 0; i < kFinFrames / 2; ++i) {
     const int fl = 2 * i + (lane >> 4);
     const int64_t f = base + fl;
     double v = 0.0;
     if (f < L.n_frames) {
       const double* part = L.partial + (size_t)f * n_tiles * kStatDoubles + (lane & 15);
+#pragma unroll 8
       for (int t = 0; t < n_tiles; ++t) v += part[(size_t)t * kStatDoubles];
     }
-    st[warp][fl][lane & 15] = v;
+    st[fl][lane & 15] = v;
   }
   __syncwarp();
   const int64_t f = base + lane;
-  if (f >= L.n_frames) return;
-  const double* tot = st[warp][lane];
-  const double W = L.ref.wsum;
-  double r[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
-  double cx[3] = {0, 0, 0}, cy[3] = {0, 0, 0};
-  if (W > 0.0 || W < 0.0) {
-    const double inv_w = 1.0 / W;
-    cx[0] = tot[0] * inv_w; cx[1] = tot[1] * inv_w; cx[2] = tot[2] * inv_w;
-    for (int c = 0; c < 3; ++c) cy[c] = ref_mean(L.ref, c);
-    if (!norotate) {
-      double h[9];
-      for (int a = 0; a < 3; ++a)
-        for (int b = 0; b < 3; ++b) h[a * 3 + b] = tot[6 + a * 3 + b] - cx[a] * ref_sum_c(L.ref, b);
-      const double gx = tot[3] + tot[4] + tot[5] - (tot[0] * cx[0] + tot[1] * cx[1] + tot[2] * cx[2]);
-      const QcpOut q = qcp_lambda(h, 0.5 * (gx + ref_gy(L.ref)));
-      rotation_from_qcp(h, q.lambda, r);
-    }
-  }
+  if (lane >= kFinFrames || f >= L.n_frames) return;
+  double r[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, t[3];
+  transform_from_totals(L.ref, st[lane], norotate, r, t);
   double* o = xf64 + f * kStatDoubles;
   for (int e = 0; e < 9; ++e) o[e] = r[e];
-  for (int i = 0; i < 3; ++i) o[9 + i] = cy[i] - (r[i * 3 + 0] * cx[0] + r[i * 3 + 1] * cx[1] + r[i * 3 + 2] * cx[2]);
+  for (int e = 0; e < 3; ++e) o[9 + e] = t[e];
   if (xf32)
     for (int e = 0; e < 12; ++e) xf32[f * 12 + e] = (float)o[e];
 }
@@ -254,8 +246,8 @@ __global__ void __launch_bounds__(kThreads, 4) superpose_apply_staged(const floa
 
 cudaError_t launch_superpose_finalize(const FrameLaunch& L, int norotate, double* xf64, float* xf32, cudaStream_t s) {
   if (L.n_frames == 0) return cudaSuccess;
-  const unsigned blocks = (unsigned)((L.n_frames + 255) / 256);
-  superpose_finalize_kernel<<<blocks, 256, 0, s>>>(L, frame_tiles(L), norotate, xf64, xf32);
+  const unsigned blocks = (unsigned)((L.n_frames + kFinFrames - 1) / kFinFrames);
+  superpose_finalize_kernel<<<blocks, 32, 0, s>>>(L, frame_tiles(L), norotate, xf64, xf32);
   return cudaGetLastError();
 }
 

@@ -99,6 +99,7 @@ struct wmd_group_ref {
   float* ref_all = nullptr;
   int64_t n_atoms = 0, n_groups = 0, n_blocks = 0;
   int64_t contig_base = -1;  // >= 0 when group_atoms[q] == contig_base + q
+  wmd::GroupStageBlocks staged;  // n 0: not consecutive atoms, or a group too large
 };
 
 struct wmd_ctx {
@@ -886,6 +887,7 @@ struct GroupJob {
   int64_t n_groups = 0;
   const float* ref_all = nullptr;
   float* out = nullptr;  // [n_frames of this call][n_groups], device
+  wmd::GroupStageBlocks staged;
 };
 
 static int superpose_device(wmd_ctx* ctx, const float* dcoords, int64_t n_frames, int64_t n_atoms, int stride,
@@ -928,7 +930,12 @@ static int superpose_device(wmd_ctx* ctx, const float* dcoords, int64_t n_frames
       CU(wmd::launch_superpose_apply(B.coords, nf, n_atoms, stride, xf, dout + (size_t)f0 * n_atoms * 3, ctx->sm_count,
                                      ctx->status_dev, s),
          "superpose apply");
-    if (grp)
+    // the staged kernel wherever its copies can run (faster at every group size it takes)
+    if (grp && grp->staged.n > 0 && stride == 3 && (reinterpret_cast<uintptr_t>(B.coords) & 15u) == 0)
+      CU(wmd::launch_group_rmsd_staged(B.coords, nf, n_atoms, xf, grp->goff, grp->contig_base, grp->staged, grp->n_groups,
+                                       grp->ref_all, grp->out + f0 * grp->n_groups, ctx->sm_count, ctx->status_dev, s),
+         "per-group rmsd");
+    else if (grp)
       CU(wmd::launch_group_rmsd(B.coords, nf, n_atoms, stride, xf, grp->goff, grp->gatoms, grp->contig_base,
                                 grp->blocks, grp->n_blocks, grp->n_groups, grp->ref_all,
                                 grp->out + f0 * grp->n_groups, ctx->sm_count, s),
@@ -1183,7 +1190,18 @@ WMD_EXPORT int wmd_group_ref_upload(wmd_ctx* ctx, const float* ref_all, int64_t 
       for (int c = 0; c < 3; ++c) ref[a * 3 + c] = raw[a * stride + c];
   }
   std::vector<uint32_t> blocks((size_t)n_groups + 1, 0);
-  const int nb = n_groups > 0 ? wmd::group_blocks(off.data(), n_groups, blocks.data()) : 0;
+  const int nb = n_groups > 0 ? wmd::group_blocks(off.data(), n_groups, blocks.data(), wmd::kGroupTile) : 0;
+  // the staged kernel's blocks: first groups and first positions
+  std::vector<uint32_t> sgroup((size_t)n_groups + 1, 0), spos;
+  int64_t ns = n_groups > 0 ? wmd::group_blocks(off.data(), n_groups, sgroup.data(), wmd::kGroupStageTile) : 0;
+  for (int64_t b = 0; b <= ns; ++b) spos.push_back(off[sgroup[b]]);
+  for (int64_t b = 0; b < ns; ++b)
+    if (spos[b + 1] - spos[b] > (uint32_t)wmd::kGroupStageTile) {
+      ns = 0;
+      break;
+    }
+  std::vector<double> inv((size_t)n_groups);
+  for (int64_t gi = 0; gi < n_groups; ++gi) inv[gi] = off[gi + 1] > off[gi] ? 1.0 / (double)(off[gi + 1] - off[gi]) : 1.0;
   wmd_group_ref* r = new wmd_group_ref();
   if (!atoms.empty()) {
     bool contig = true;
@@ -1200,7 +1218,9 @@ WMD_EXPORT int wmd_group_ref_upload(wmd_ctx* ctx, const float* ref_all, int64_t 
     return at;
   };
   const size_t o_off = take(off.size() * 4), o_atoms = take(std::max<size_t>(atoms.size(), 1) * 4),
-               o_blocks = take(((size_t)nb + 1) * 4), o_ref = take(std::max<size_t>(ref.size(), 1) * 4);
+               o_blocks = take(((size_t)nb + 1) * 4), o_spos = take(((size_t)ns + 1) * 4),
+               o_sgroup = take(((size_t)ns + 1) * 4), o_inv = take(std::max<size_t>((size_t)n_groups, 1) * 8),
+               o_ref = take(std::max<size_t>(ref.size(), 1) * 4);
   cudaError_t e = cudaMalloc(&r->mem, total);
   if (e != cudaSuccess) {
     delete r;
@@ -1212,9 +1232,19 @@ WMD_EXPORT int wmd_group_ref_upload(wmd_ctx* ctx, const float* ref_all, int64_t 
   r->gatoms = reinterpret_cast<uint32_t*>(base + o_atoms);
   r->blocks = reinterpret_cast<uint32_t*>(base + o_blocks);
   r->ref_all = reinterpret_cast<float*>(base + o_ref);
+  uint32_t* d_spos = reinterpret_cast<uint32_t*>(base + o_spos);
+  uint32_t* d_sgroup = reinterpret_cast<uint32_t*>(base + o_sgroup);
+  double* d_inv = reinterpret_cast<double*>(base + o_inv);
+  r->staged.pos = d_spos;
+  r->staged.group = d_sgroup;
+  r->staged.inv_count = d_inv;
+  r->staged.n = r->contig_base >= 0 ? ns : 0;
   e = cudaMemcpy(r->goff, off.data(), off.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && !atoms.empty()) e = cudaMemcpy(r->gatoms, atoms.data(), atoms.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(r->blocks, blocks.data(), ((size_t)nb + 1) * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d_spos, spos.data(), ((size_t)ns + 1) * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && n_groups > 0) e = cudaMemcpy(d_inv, inv.data(), inv.size() * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d_sgroup, sgroup.data(), ((size_t)ns + 1) * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && !ref.empty()) e = cudaMemcpy(r->ref_all, ref.data(), ref.size() * 4, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(r->mem);
@@ -1276,6 +1306,7 @@ WMD_EXPORT int wmd_rmsd_per_group(wmd_ctx* ctx, const float* coords, int64_t n_f
   job.contig_base = groups->contig_base;
   job.n_groups = n_groups;
   job.ref_all = groups->ref_all;
+  job.staged = groups->staged;
   const bool oh = is_host(classify(out));
   const size_t row = (size_t)n_groups * sizeof(float);
   rc = for_each_chunk(ctx, coords, n_frames, n_atoms, stride, s, [&](const float* dc, int64_t f0, int64_t nf) -> int {
