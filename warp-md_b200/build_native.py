@@ -19,8 +19,8 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 OUT_DIR = os.path.join(HERE, "warp_md", "_native")
 LIB = os.path.join(OUT_DIR, "libwarpmd_rmsd.so")
-SOURCES = ["wmd_api.cu", "rmsd_frames.cu", "rmsd_lanes.cu", "rmsd_vg.cu", "pairwise.cu", "pairwise_tc.cu", "pairwise_tc64.cu", "pairwise_dme.cu", "noalloc.cu", "batched.cu", "superpose.cu", "fluct.cu", "cluster.cu", "dcd.cu", "reference.cu"]
-HEADERS = ["device_util.cuh", "frame_parts.cuh", "tcgen05.cuh", "tile_walk.h", "qcp.cuh", "wmd_internal.h", "pairwise.h", "pairwise_tc.h", "pairwise_dme.h", "batched.h", "superpose.h", "fluct.h", "cluster.h", "dcd.h"]
+SOURCES = ["wmd_api.cu", "rmsd_frames.cu", "frame_small.cu", "rmsd_lanes.cu", "rmsd_vg.cu", "pairwise.cu", "pairwise_tc.cu", "pairwise_tc64.cu", "pairwise_dme.cu", "noalloc.cu", "batched.cu", "superpose.cu", "fluct.cu", "cluster.cu", "dcd.cu", "reference.cu"]
+HEADERS = ["device_util.cuh", "frame_parts.cuh", "frame_residual.cuh", "tcgen05.cuh", "tile_walk.h", "qcp.cuh", "wmd_internal.h", "pairwise.h", "pairwise_tc.h", "pairwise_dme.h", "batched.h", "superpose.h", "fluct.h", "cluster.h", "dcd.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

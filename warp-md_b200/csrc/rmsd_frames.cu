@@ -40,6 +40,7 @@
 
 #include "device_util.cuh"
 #include "frame_parts.cuh"
+#include "frame_residual.cuh"
 #include "qcp.cuh"
 #include "wmd_internal.h"
 
@@ -364,76 +365,23 @@ __global__ void __launch_bounds__(kThreads, 3) rmsd_frames_kernel(const FrameLau
   }
 }
 
-// Backward prologue: per frame, the rotation from the QCP eigenvector of the
-// stored H, the centroid and the scale dL/drmsd / (n rmsd).
+// Backward prologue: every frame's rotation record.
 __global__ void rmsd_bwd_prologue(const double* __restrict__ stats, const float* __restrict__ grad_rmsd,
                                   const double* __restrict__ grad_f64, int64_t grad_stride, int64_t n_frames,
                                   double* __restrict__ rot) {
   const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= n_frames) return;
-  const double* st = stats + f * kStatDoubles;
-  double h[9], r[9];
-  for (int e = 0; e < 9; ++e) h[e] = st[3 + e];
-  rotation_from_qcp(h, st[12], r);
-  const double rmsd = st[13], n = st[14];
-  const double g = grad_f64 ? grad_f64[f * grad_stride] : grad_rmsd ? (double)grad_rmsd[f] : 1.0;
-  const double scale = (rmsd > 0.0 && n > 0.0) ? g / (n * rmsd) : 0.0;
-  double* o = rot + f * kStatDoubles;
-  for (int e = 0; e < 9; ++e) o[e] = r[e];
-  o[9] = st[0]; o[10] = st[1]; o[11] = st[2];
-  o[12] = scale; o[13] = 0; o[14] = 0; o[15] = 0;
+  frame_rotation(stats, grad_rmsd, grad_f64, grad_stride, f, rot + f * kStatDoubles);
 }
 
-// Residual pass for flagged frames (near-zero RMSD): the RMSD from explicit
-// residuals sum |R (x_k - x_bar) - (y_k - y_bar)|^2 in FP64, as the reference's
-// rmsd_aligned_selected computes every frame (plan.rs:1223-1247), with R from
-// the QCP eigenvector.  One CTA per flagged frame (grid-stride).
+// Residual pass for flagged frames (near-zero RMSD).  One CTA per flagged frame
+// (grid-stride).
 template <int STRIDE>
 __global__ void __launch_bounds__(256) rmsd_refine_kernel(const FrameLaunch L) {
-  __shared__ double sh_r[12];
   __shared__ double red[8];
   const unsigned count = *L.refine_count;
-  const int64_t n_sel = L.ref.n_sel;
-  const double inv_n = 1.0 / (double)n_sel;
   for (unsigned rix = blockIdx.x; rix < count; rix += gridDim.x) {
-    const double* rec = L.refine + (size_t)rix * kStatDoubles;
-    if (threadIdx.x == 0) {
-      double h[9], r[9];
-      for (int e = 0; e < 9; ++e) h[e] = rec[4 + e];
-      rotation_from_qcp(h, rec[13], r);
-      for (int e = 0; e < 9; ++e) sh_r[e] = r[e];
-      sh_r[9] = rec[1]; sh_r[10] = rec[2]; sh_r[11] = rec[3];
-    }
-    __syncthreads();
-    const int64_t f = (int64_t)rec[0];
-    double R[9], c[3];
-    for (int e = 0; e < 9; ++e) R[e] = sh_r[e];
-    c[0] = sh_r[9]; c[1] = sh_r[10]; c[2] = sh_r[11];
-    const double my0 = ref_sum_c(L.ref, 0) * inv_n, my1 = ref_sum_c(L.ref, 1) * inv_n,
-                 my2 = ref_sum_c(L.ref, 2) * inv_n;
-    const float* frame = L.coords + (size_t)f * L.n_atoms * STRIDE;
-    double acc = 0.0;
-    for (int64_t k = threadIdx.x; k < n_sel; k += blockDim.x) {
-      int64_t atom = L.sel ? (int64_t)L.sel[k] : k;
-      if (atom >= L.n_atoms) atom = 0;  // reported by the forward kernel
-      const float* p = frame + atom * STRIDE;
-      const double d0 = (double)p[0] - c[0], d1 = (double)p[1] - c[1], d2 = (double)p[2] - c[2];
-      const double* y = L.ref.yc + k * 3;
-      const double r0 = R[0] * d0 + R[1] * d1 + R[2] * d2 - (y[0] - my0);
-      const double r1 = R[3] * d0 + R[4] * d1 + R[5] * d2 - (y[1] - my1);
-      const double r2 = R[6] * d0 + R[7] * d1 + R[8] * d2 - (y[2] - my2);
-      acc += r0 * r0 + r1 * r1 + r2 * r2;
-    }
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < 8; ++w) t += red[w];
-      const double rmsd = sqrt(t * inv_n);
-      if (L.out.rmsd) L.out.rmsd[f] = rmsd;
-      if (L.out.stats) L.out.stats[f * kStatDoubles + 13] = rmsd;
-    }
+    residual_rmsd<STRIDE>(L, L.refine + (size_t)rix * kStatDoubles, red);
     __syncthreads();
   }
 }
@@ -583,6 +531,7 @@ int frame_grid(const FrameLaunch& L, int sm_count, bool backward) {
 
 cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s) {
   if (L.n_frames == 0) return cudaSuccess;
+  if (small_frames(L)) return launch_small_forward(L, s);
   FrameLaunch K = L;
   // few tiles per frame: the frames-across-lanes kernel finishes its frames itself
   const bool fused = L.lanes && L.group_done && frame_tiles(L) <= kLaneFinishTiles && L.n_frames >= 4;
@@ -637,6 +586,7 @@ cudaError_t launch_rmsd_stream_weighted(const FrameLaunch& L, cudaStream_t s) {
 cudaError_t launch_rmsd_backward(const FrameLaunch& L, const double* stats, const float* grad_rmsd,
                                  const double* grad_f64, int64_t grad_stride, double* rot_scratch, cudaStream_t s) {
   if (L.n_frames == 0) return cudaSuccess;
+  if (small_frames(L)) return launch_small_backward(L, stats, grad_rmsd, grad_f64, grad_stride, s);
   const int threads = 128;
   const int blocks = (int)((L.n_frames + threads - 1) / threads);
   rmsd_bwd_prologue<<<blocks, threads, 0, s>>>(stats, grad_rmsd, grad_f64, grad_stride, L.n_frames, rot_scratch);

@@ -114,6 +114,11 @@ constexpr int kLaneFinishTiles = 16;
 // Forward: zeroes L.refine_count, runs the fused kernel, then the residual pass
 // over the frames it flagged.
 cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s);
+// Launches too small to fill the GPU: one CTA per frame, one launch (frame_small.cu).
+bool small_frames(const FrameLaunch& L);
+cudaError_t launch_small_forward(const FrameLaunch& L, cudaStream_t s);
+cudaError_t launch_small_backward(const FrameLaunch& L, const double* stats, const float* grad_rmsd,
+                                  const double* grad_f64, int64_t grad_stride, cudaStream_t s);
 // Only the streaming kernel of the aligned forward (tile partials into
 // L.partial); the caller finishes the frames itself.
 cudaError_t launch_rmsd_stream(const FrameLaunch& L, cudaStream_t s);
