@@ -82,7 +82,7 @@ __device__ __forceinline__ void transform_from_totals(const RefInfo& ref, const 
 }
 
 // Positions per lane whose loads are in flight together in gather_item.
-constexpr int kGatherJ = 4;
+constexpr int kGatherDepth = 4;
 
 // An atom's 12 bytes cost two loads, not three: an 8-byte load of the pair
 // that starts on an 8-byte boundary (x,y or y,z) and a 4-byte load of the
@@ -97,15 +97,26 @@ __device__ __forceinline__ void load_xyz(const float* p, float& x, float& y, flo
 }
 
 // One warp's sums over list positions [a0, a1) of a frame (L.sel's atoms, or the
-// positions themselves), in sub-chunks of 32 x kGatherJ positions with all of a
+// positions themselves; kDense: there is no list), in sub-chunks of 32 x kGatherJ positions with all of a
 // sub-chunk's loads in flight before any use.  Returned as
 // warp_reduce_scatter16 leaves them: lane 2e holds sum e.
-template <int STRIDE, int MODE>
+template <int STRIDE, int MODE, int kGatherJ = kGatherDepth, bool kDense = false>
 __device__ __forceinline__ double gather_item(const FrameLaunch& L, const float* __restrict__ frame, int64_t a0,
                                               int64_t a1, const double (&mean)[3], int lane) {
   double acc[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) acc[e] = 0.0;
+  // the next sub-chunk's indices are loaded a sub-chunk ahead, so that its atoms' loads
+  // do not wait for them
+  uint32_t next[kGatherJ];
+  auto fetch = [&](int64_t c0) {
+#pragma unroll
+    for (int j = 0; j < kGatherJ; ++j) {
+      const int64_t k = c0 + lane + 32 * j;
+      if (!kDense && L.sel && k < a1) next[j] = __ldg(L.sel + k);
+    }
+  };
+  fetch(a0);
 #pragma unroll 1
   for (int64_t c0 = a0; c0 < a1; c0 += 32 * kGatherJ) {
     float x[kGatherJ][3];
@@ -115,8 +126,8 @@ __device__ __forceinline__ double gather_item(const FrameLaunch& L, const float*
     for (int j = 0; j < kGatherJ; ++j) {
       const int64_t k = c0 + lane + 32 * j;
       if (k < a1) {
-        int64_t idx = L.sel ? (int64_t)__ldg(L.sel + k) : k;
-        if (idx >= L.n_atoms) {  // bad device-side selection: report, read atom 0
+        int64_t idx = !kDense && L.sel ? (int64_t)next[j] : k;
+        if (!kDense && idx >= L.n_atoms) {  // bad device-side selection: report, read atom 0
           atomicOr(L.status, kStatusBadIndex);
           idx = 0;
         }
@@ -130,6 +141,7 @@ __device__ __forceinline__ double gather_item(const FrameLaunch& L, const float*
         if (MODE == kFwdW) wt[MODE == kFwdW ? j : 0] = 0.f;
       }
     }
+    fetch(c0 + 32 * kGatherJ);
 #pragma unroll
     for (int j = 0; j < kGatherJ; ++j) {
       const double x0 = x[j][0], x1 = x[j][1], x2 = x[j][2];

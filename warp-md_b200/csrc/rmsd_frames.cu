@@ -387,18 +387,25 @@ __global__ void __launch_bounds__(256) rmsd_refine_kernel(const FrameLaunch L) {
 }
 
 // Gathered forward statistics (a selection's scattered atoms, or frames whose
-// base is not 16-byte aligned).  One warp per (tile, frame) item, tiles of
-// kConsumerThreads * kApt list positions as in the streaming kernel, so the
-// partial records and rmsd_finalize_kernel are shared.  No block barrier: a
+// base is not 16-byte aligned).  One warp per (tile, frame) item; the partial records
+// and rmsd_finalize_kernel are the streaming kernel's.  No block barrier: a
 // warp walks its contiguous run of items (tile-major, so a tile's indices and
-// reference stay in L1 across frames) in sub-chunks of 32 x kGatherJ
+// reference stay in L1 across frames) in sub-chunks of 32 x gather_depth
 // positions, all of a sub-chunk's loads in flight before any use, and
-// reduces its sums with shuffles.  Latency is hidden by the warps resident
-// per SM instead of by a CTA-wide pipeline.
+// reduces its sums with shuffles.  Bound by the latency of those loads until HBM
+// is (every tenth atom already fetches the whole frame): resident warps count for
+// more than loads per warp, as long as nothing spills.  Measured, with the tile
+// chosen by gather_tile, 1,000 x 100,000 every tenth / 2,000 x 20,000 every second
+// atom: 4 positions a lane, 4 CTAs an SM 195 / 202 us; 2 and 6: 193 / 153; 2 and 5
+// 194 / 167; 1 and 8 196 / 140.  With weights (superpose, 1,000 x 100,000): 606 us
+// the call with 4 and 4, 612 with 2 and 6 (spills), 621 with 1 and 8.  Before (4 and
+// 4, indices loaded with their atoms, 1,024-position tiles): 222 / 248 us.
 constexpr int kGatherThreads = 128;
+constexpr int gather_depth(int mode) { return mode == kFwdW ? 4 : 2; }
+constexpr int gather_ctas(int mode) { return mode == kFwdW ? 4 : 6; }
 
 template <int STRIDE, int MODE>
-__global__ void __launch_bounds__(kGatherThreads) rmsd_gather_kernel(const FrameLaunch L, int tile) {
+__global__ void __launch_bounds__(kGatherThreads, gather_ctas(MODE)) rmsd_gather_kernel(const FrameLaunch L, int tile) {
   const int lane = threadIdx.x & 31;
   const int64_t gw = ((int64_t)blockIdx.x * kGatherThreads + threadIdx.x) >> 5;
   const int64_t n_warps = (int64_t)gridDim.x * (kGatherThreads / 32);
@@ -415,7 +422,7 @@ __global__ void __launch_bounds__(kGatherThreads) rmsd_gather_kernel(const Frame
     const int64_t a0 = (int64_t)t * tile;
     const int64_t a1 = min(n_sel, a0 + tile);
     const float* frame = L.coords + (size_t)f * L.n_atoms * STRIDE;
-    const double v = gather_item<STRIDE, MODE>(L, frame, a0, a1, mean, lane);
+    const double v = gather_item<STRIDE, MODE, gather_depth(MODE)>(L, frame, a0, a1, mean, lane);
     if ((lane & 1) == 0) L.partial[((size_t)f * n_tiles + t) * kStatDoubles + (lane >> 1)] = v;
     if (++f == F) { f = 0; ++t; }
   }
@@ -431,12 +438,12 @@ static cudaError_t launch_gather(const FrameLaunch& L, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <int STRIDE>
+template <int STRIDE, int MODE>
 static int gather_occupancy() {
   int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, rmsd_gather_kernel<STRIDE, kFwdW>, kGatherThreads, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, rmsd_gather_kernel<STRIDE, MODE>, kGatherThreads, 0) !=
       cudaSuccess)
-    blocks = 4;
+    blocks = gather_ctas(MODE);
   return blocks < 1 ? 1 : blocks;
 }
 
@@ -498,6 +505,36 @@ size_t frame_smem_bytes(int stride, int tile_atoms) {
   return stride == 4 ? Geo<4, kApt>::kSmemBytes : Geo<3, kApt>::kSmemBytes;
 }
 
+// Resident warps of the gathered kernel.
+static int64_t gather_slots(const FrameLaunch& L, int sm_count) {
+  static int cache[2][2] = {};  // [stride4][weighted]
+  int& occ = cache[L.stride == 4][L.ref.w != nullptr];
+  if (occ == 0) {
+    if (L.ref.w) occ = L.stride == 4 ? gather_occupancy<4, kFwdW>() : gather_occupancy<3, kFwdW>();
+    else occ = L.stride == 4 ? gather_occupancy<4, kFwdFit>() : gather_occupancy<3, kFwdFit>();
+  }
+  return (int64_t)sm_count * occ * (kGatherThreads / 32);
+}
+
+// Tile of the gathered kernel, a multiple of 128 list positions up to 1,024,
+// minimising the busiest warp's work: (items per warp) x (tile + an item's fixed
+// part, its reduction and record, worth about 96 positions).  600 x 10,000 every
+// tenth (600 items of one 1,000-position tile) 44 -> 26 us, 1,000 x 100,000 (2.4 items
+// a warp) 222 -> 207 us.
+static int gather_tile(const FrameLaunch& L, int sm_count) {
+  const int64_t slots = gather_slots(L, sm_count);
+  int64_t best = 1024, best_cost = -1;
+  for (int64_t tile = 1024; tile >= 128; tile -= 128) {
+    const int64_t items = (L.ref.n_sel + tile - 1) / tile * L.n_frames;
+    const int64_t cost = (items + slots - 1) / slots * (std::min(tile, L.ref.n_sel) + 96);
+    if (best_cost < 0 || cost < best_cost) {
+      best = tile;
+      best_cost = cost;
+    }
+  }
+  return (int)best;
+}
+
 void frame_plan(FrameLaunch& L, int sm_count) {
   // a dense selection streams itself; a gathered one only through an
   // expansion the caller prepared (lane_y set)
@@ -509,17 +546,15 @@ void frame_plan(FrameLaunch& L, int sm_count) {
   }
   L.lanes = L.lane_y && lanes_eligible(L) && lanes_worthwhile(L, sm_count);
   L.tile_atoms = L.lanes ? lanes_tile(L, sm_count) : kConsumerThreads * kApt;
+  if (!L.lanes && L.gather) L.tile_atoms = gather_tile(L, sm_count);
 }
 
 int frame_grid(const FrameLaunch& L, int sm_count, bool backward) {
   if (L.lanes && !backward) return lanes_grid(L, sm_count);
   if (L.gather && !backward) {
-    static int gocc[2] = {};
-    int& occ = gocc[L.stride == 4];
-    if (occ == 0) occ = L.stride == 4 ? gather_occupancy<4>() : gather_occupancy<3>();
     const int64_t warps = (int64_t)frame_tiles(L) * L.n_frames;  // one warp per item at most
-    const int64_t cap = (int64_t)sm_count * occ;
-    return (int)std::max<int64_t>(1, std::min<int64_t>((warps + kGatherThreads / 32 - 1) / (kGatherThreads / 32), cap));
+    const int64_t n = std::min(warps, gather_slots(L, sm_count));
+    return (int)std::max<int64_t>(1, (n + kGatherThreads / 32 - 1) / (kGatherThreads / 32));
   }
   static int cache[2][2][2] = {};  // [bwd][stride4][gather]
   int& occ = cache[backward ? 1 : 0][L.stride == 4][L.gather ? 1 : 0];

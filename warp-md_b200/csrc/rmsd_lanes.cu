@@ -278,8 +278,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
     for (int64_t t = warps - 1 - gw; t < n_tiles; t += warps) {
       for (int64_t f = F; f < F + L.tail_frames; ++f) {
         const int64_t a0 = t * tile, a1 = min(n_sel, a0 + tile);
-        const double v = gather_item<3, RAW ? kFwdRaw : (W ? kFwdW : kFwdFit)>(L, L.coords + (size_t)f * L.n_atoms * 3, a0,
-                                                                             a1, mean, lane);
+        const double v = gather_item<3, RAW ? kFwdRaw : (W ? kFwdW : kFwdFit), kGatherDepth, true>(
+            L, L.coords + (size_t)f * L.n_atoms * 3, a0, a1, mean, lane);
         if ((lane & 1) == 0) L.partial[((size_t)f * n_tiles + t) * kStatDoubles + (lane >> 1)] = v;
       }
       if (L.group_done && last_of_group(groups) && lane < L.tail_frames) finish_from_records(F + lane);
