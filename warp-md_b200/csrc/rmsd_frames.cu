@@ -496,8 +496,8 @@ static int occupancy(const FrameLaunch& L) {
 }
 
 int frame_tiles(const FrameLaunch& L) {
-  const int64_t n = L.lanes ? L.lane_atoms : L.ref.n_sel;
-  return (int)((n + L.tile_atoms - 1) / L.tile_atoms);
+  if (L.lanes) return 1;  // it leaves a frame's sums, or nothing
+  return (int)((L.ref.n_sel + L.tile_atoms - 1) / L.tile_atoms);
 }
 
 size_t frame_smem_bytes(int stride, int tile_atoms) {
@@ -545,8 +545,7 @@ void frame_plan(FrameLaunch& L, int sm_count) {
     L.lane_w = L.ref.w;
   }
   L.lanes = L.lane_y && lanes_eligible(L) && lanes_worthwhile(L, sm_count);
-  L.tile_atoms = L.lanes ? lanes_tile(L, sm_count) : kConsumerThreads * kApt;
-  if (!L.lanes && L.gather) L.tile_atoms = gather_tile(L, sm_count);
+  L.tile_atoms = !L.lanes && L.gather ? gather_tile(L, sm_count) : kConsumerThreads * kApt;
 }
 
 int frame_grid(const FrameLaunch& L, int sm_count, bool backward) {
@@ -568,19 +567,18 @@ cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s) {
   if (L.n_frames == 0) return cudaSuccess;
   if (small_frames(L)) return launch_small_forward(L, s);
   FrameLaunch K = L;
-  // few tiles per frame: the frames-across-lanes kernel finishes its frames itself
-  const bool fused = L.lanes && L.group_done && frame_tiles(L) <= kLaneFinishTiles && L.n_frames >= 4;
-  if (!fused) K.group_done = nullptr;
   const bool refine = L.align && L.refine;
   cudaError_t e = cudaSuccess;
-  const size_t done_bytes = fused ? (size_t)frame_groups(L.n_frames) * sizeof(unsigned) : 0;
-  if (refine) e = cudaMemsetAsync(L.refine_count, 0, sizeof(unsigned) + done_bytes, s);
-  else if (fused) e = cudaMemsetAsync(L.group_done, 0, done_bytes, s);
-  if (e != cudaSuccess) return e;
-  if (L.align) e = L.lanes ? launch_lanes_forward(K, false, s) : dispatch<kFwdFit>(K, s);
-  else e = L.lanes ? launch_lanes_forward(K, true, s) : dispatch<kFwdRaw>(K, s);
-  if (e != cudaSuccess) return e;
-  if (!fused) {
+  if (refine) {  // and the counters behind it
+    const size_t done = L.lanes ? (size_t)frame_groups(L.n_frames) : 0;
+    e = cudaMemsetAsync(L.refine_count, 0, (1 + done) * sizeof(unsigned), s);
+    K.done_cleared = L.lanes;
+    if (e != cudaSuccess) return e;
+  }
+  if (L.lanes) {
+    if ((e = launch_lanes_forward(K, !L.align, s)) != cudaSuccess) return e;
+  } else {
+    if ((e = L.align ? dispatch<kFwdFit>(K, s) : dispatch<kFwdRaw>(K, s)) != cudaSuccess) return e;
     const unsigned blocks = (unsigned)((L.n_frames + 7) / 8);
     if (L.align) rmsd_finalize_kernel<kFwdFit><<<blocks, 256, 0, s>>>(K, frame_tiles(L));
     else rmsd_finalize_kernel<kFwdRaw><<<blocks, 256, 0, s>>>(K, frame_tiles(L));
@@ -591,21 +589,6 @@ cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s) {
   if (L.stride == 4) rmsd_refine_kernel<4><<<blocks, 256, 0, s>>>(K);
   else rmsd_refine_kernel<3><<<blocks, 256, 0, s>>>(K);
   return cudaGetLastError();
-}
-
-cudaError_t launch_gather_partials(const FrameLaunch& L, bool raw, int sm_count, cudaStream_t s) {
-  if (L.n_frames == 0) return cudaSuccess;
-  FrameLaunch B = L;
-  B.lanes = false;
-  B.gather = true;
-  B.grid = frame_grid(B, sm_count, false);
-  const int mode = raw ? kFwdRaw : (L.ref.w ? kFwdW : kFwdFit);
-  if (L.stride == 4) {
-    if (mode == kFwdRaw) return launch_gather<4, kFwdRaw>(B, s);
-    return mode == kFwdW ? launch_gather<4, kFwdW>(B, s) : launch_gather<4, kFwdFit>(B, s);
-  }
-  if (mode == kFwdRaw) return launch_gather<3, kFwdRaw>(B, s);
-  return mode == kFwdW ? launch_gather<3, kFwdW>(B, s) : launch_gather<3, kFwdFit>(B, s);
 }
 
 cudaError_t launch_rmsd_stream(const FrameLaunch& L, cudaStream_t s) {

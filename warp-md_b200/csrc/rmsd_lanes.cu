@@ -13,12 +13,22 @@
 //     by lane 0 as soon as the warp is done with one.
 //   * Each lane adds, in FP64 and in atom order, the 15 sums of its own frame
 //     (sum x, sum x_a^2, sum x y_c^T): no shuffles, no barriers.
-//   * Atoms are grouped into tiles (128 to 2,048 atoms, chosen per launch so
-//     that whole units balance over the warp slots); a unit is (tile,
-//     32-frame group) and belongs to one warp, which stores each lane's 16 sums into
-//     the same [frame][tile][16] partials the finalize kernel reads.  Every
-//     warp gets the same number of whole units, so results do not depend on
-//     the launch shape and are bitwise reproducible.
+//   * The stages of all frame groups, group after group, are split over the
+//     warp slots in equal runs (LaneSplit).  A group within one run is finished from
+//     registers; otherwise each of its warps stores a record (15 sums x 32 frames,
+//     coalesced, in L2) and the last to do so adds them in warp order and finishes
+//     the group, a frame per lane, while other warps still stream.  The split depends
+//     on the sizes and the device alone, so results are bitwise reproducible.
+//     With more than kLaneFinishParts warps a group (few frames of many atoms),
+//     lanes_finalize_kernel adds the records, a CTA a group.
+//
+// Whole (tile, group) units, tile after tile, used to be the warps' work: the last tile's
+// few warps then finished every group (31 us for 2,400 x 1,000, whose stream takes
+// 4.4), a warp had 1 or 2 units but not 1.5, and the records were a frame apart.
+// Measured, us a call, then / with equal runs: 2,400 x 4,000 58 / 37; 5,000 x 8,000
+// 119 / 94; 20,000 x 3,000 209 / 132; 5,001 x 3,001 62 / 50; 2,000 x 20,000 101 / 96.
+// Bound by HBM for long runs (4,000 x 100,000: 6.5 TB/s); short ones by the launch,
+// the first loads and the finish (~12 us together).
 //
 // Frames whose stride is not a multiple of 16 bytes (packed xyz with
 // n_atoms % 4 != 0) cannot be rows of a tensor map; four consecutive frames
@@ -30,17 +40,9 @@
 // rows of 400 bytes put the 32 lanes in distinct banks for odd n_atoms (two
 // lanes per bank otherwise).  Atoms past the tile come from the next frame of
 // the quad row and are masked.  The last n_frames mod 4 frames are no quad row:
-// their tiles are summed with plain loads, atoms across lanes, by the last warps
-// of the grid (those without units of their own, where there are any) before
-// their units.  As a launch behind this kernel they cost 12 us of 83 for 5,001
+// their tiles are summed with plain loads, atoms across lanes, by warps set aside
+// for them.  As a launch behind this kernel they cost 12 us of 83 for 5,001
 // frames x 3,001 atoms.
-//
-// Finishing.  With L.group_done set, the warp that stores a frame group's last
-// tile adds the group's tiles in tile order and runs QCP, one frame per lane,
-// while other warps still stream: the separate finalize kernel (a warp per frame,
-// QCP on one lane) took 16 us of those 83.  Up to kLaneFinishTiles tiles: a lane
-// reads its frame's records one after another, so with hundreds of them the
-// finalize kernel, a warp per frame, is ahead.
 //
 // Atoms streamed: a dense selection (the first n_sel atoms), or the span
 // [lane_atom0, lane_atom0 + lane_atoms) of a sorted selection with the
@@ -70,6 +72,13 @@ namespace {
 constexpr int kLaneWarps = 4;   // warps per CTA
 constexpr int kLaneStages = 2;  // stage ring per warp
 constexpr int kLaneAtoms = 32;  // atoms per stage
+constexpr int kLaneBlock = 16;  // stages added up in one chain
+// The split of the stages over the warps (lanes_split): fewest stages a warp, most
+// stages that runs of whole groups may add to the busiest warp, most parts of a group
+// that the last of its warps adds up itself.
+constexpr int kLaneMinStages = 4;
+constexpr int kLaneWholeStages = 4;
+constexpr int kLaneFinishParts = 16;
 
 template <int STRIDE>
 struct LaneGeo {
@@ -214,6 +223,55 @@ __device__ __forceinline__ void stage_sums_quad(double (&acc)[15], const unsigne
   }
 }
 
+// How the frame groups' stages are split over the active warps: group-major, in
+// equal runs (lane_whole: runs of whole groups).  A warp's run holds whole groups
+// and at most two parts of groups, its first and its last, each with a record of
+// 15 sums x 32 frames.
+struct LaneSplit {
+  int64_t nw, groups, total;
+  int stages;
+  bool whole;
+  __device__ __forceinline__ explicit LaneSplit(const FrameLaunch& L)
+      : nw(L.lane_warps), groups((L.n_frames + 31) / 32), stages((int)((L.lane_atoms + kLaneAtoms - 1) / kLaneAtoms)),
+        whole(L.lane_whole) {
+    total = groups * stages;
+  }
+  // first stage of warp w's run
+  __device__ __forceinline__ int64_t first(int64_t w) const {
+    return whole ? groups * w / nw * stages : total * w / nw;
+  }
+  // warp whose run holds stage j (not with whole)
+  __device__ __forceinline__ int64_t owner(int64_t j) const { return ((j + 1) * nw - 1) / total; }
+  __device__ __forceinline__ double* record(const FrameLaunch& L, int64_t w, int64_t g) const {
+    return L.lane_rec + (2 * w + (first(w) >= g * stages ? 0 : 1)) * (16 * 32);
+  }
+  // tot = the records of group g of warps wa, wa + step, ... below wb, in that order
+  template <int UNROLL>
+  __device__ __forceinline__ void add_records(const FrameLaunch& L, int64_t g, int64_t wa, int64_t wb, int step, int lane,
+                                              double (&tot)[16]) const {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) tot[e] = 0.0;
+#pragma unroll UNROLL
+    for (int64_t w = wa; w < wb; w += step) {
+      // the warp that holds the group's start may have another group's part first
+      const double* rec = record(L, w, g) + lane;
+#pragma unroll
+      for (int e = 0; e < 15; ++e) tot[e] += __ldcg(rec + e * 32);
+    }
+  }
+};
+
+// A frame's outputs, or its sums for a caller that finishes the frames itself.
+__device__ __forceinline__ void lane_finish(const FrameLaunch& L, int64_t f, const double (&tot)[16], int mode) {
+  if (!L.lane_totals) {
+    finish_totals(L, f, tot, mode);
+    return;
+  }
+  double2* o = reinterpret_cast<double2*>(L.partial + f * kStatDoubles);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) o[e] = make_double2(tot[2 * e], tot[2 * e + 1]);
+}
+
 template <int STRIDE, bool RAW, bool W, bool QUAD = false>
 __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __grid_constant__ CUtensorMap map,
                                                                      const FrameLaunch L) {
@@ -230,11 +288,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
   // selection covers (L.lane_atom0 is folded into the tensor map's base)
   const int64_t F = L.n_frames, n_sel = L.lane_atoms;
   const int64_t groups = (F + 31) / 32;
-  const int64_t tile = L.tile_atoms;  // a multiple of kLaneAtoms
-  const int n_tiles = (int)((n_sel + tile - 1) / tile);
-  const int64_t units = groups * n_tiles;  // (tile, frame group), tile-major
   const int64_t nw = L.lane_warps, gw = (int64_t)blockIdx.x * kLaneWarps + warp;
-  const int64_t u0 = units * gw / nw, u1 = units * (gw + 1) / nw;
+  const LaneSplit split(L);
   constexpr int kMode = RAW ? kFwdRaw : kFwdFit;
   const double mean[3] = {RAW ? ref_mean(L.ref, 0) : 0.0, RAW ? ref_mean(L.ref, 1) : 0.0, RAW ? ref_mean(L.ref, 2) : 0.0};
 
@@ -245,64 +300,62 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
   }
   __syncthreads();
 
-  // this warp has stored its records of group g's tile (lane: frame f, if any):
-  // true when they were the last of the group's
-  auto last_of_group = [&](int64_t g) {
+  // counts this warp's stored records of one of `parts` parts: true for the last
+  auto last_part = [&](int64_t counter, int parts) {
     __threadfence();
     __syncwarp();
     unsigned before = 0;
-    if (lane == 0) before = atomicAdd(L.group_done + g, 1u);
+    if (lane == 0) before = atomicAdd(L.group_done + counter, 1u);
     before = __shfl_sync(0xffffffffu, before, 0);
-    if (before + 1u != (unsigned)n_tiles) return false;
+    if (before + 1u != (unsigned)parts) return false;
     __threadfence();
     return true;
   };
-  auto finish_from_records = [&](int64_t f) {
-    const double2* rec = reinterpret_cast<const double2*>(L.partial + (size_t)f * n_tiles * kStatDoubles);
+
+  if (gw >= nw) {
+    // the frames past the last quad row, by warps of their own: (frame, tile) items
+    const int64_t item = gw - nw, tiles = (n_sel + L.lane_tail_tile - 1) / L.lane_tail_tile;
+    if (!QUAD || item >= L.tail_frames * tiles) return;
+    double* tail = L.lane_rec + 2 * nw * (16 * 32);  // [tail frame][tile][16]
+    const int64_t t = item % tiles;
+    const double v = gather_item<3, RAW ? kFwdRaw : (W ? kFwdW : kFwdFit), kGatherDepth, true>(
+        L, L.coords + (size_t)(F + item / tiles) * L.n_atoms * 3, t * L.lane_tail_tile,
+        min(n_sel, (t + 1) * L.lane_tail_tile), mean, lane);
+    if ((lane & 1) == 0) tail[item * 16 + (lane >> 1)] = v;
+    if (!last_part(groups, L.lane_tail_warps)) return;
+    // a lane per (element, parity) adds the tiles of a frame, then lane k finishes frame k
     double tot[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) tot[e] = 0.0;
-#pragma unroll 2
-    for (int t = 0; t < n_tiles; ++t)
+    for (int k = 0; k < L.tail_frames; ++k) {
+      double s = 0.0;
+#pragma unroll 8
+      for (int64_t i = lane >> 4; i < tiles; i += 2) s += __ldcg(tail + (k * tiles + i) * 16 + (lane & 15));
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const double2 v = __ldcg(rec + t * 8 + e);
-        tot[2 * e] += v.x;
-        tot[2 * e + 1] += v.y;
+      for (int e = 0; e < 16; ++e) {
+        const double v = __shfl_sync(0xffffffffu, s, e);
+        if (lane == k) tot[e] = v;
       }
-    finish_totals(L, f, tot, kMode);
-  };
-
-  if (QUAD && L.tail_frames > 0) {
-    const int64_t warps = (int64_t)gridDim.x * kLaneWarps;
-    for (int64_t t = warps - 1 - gw; t < n_tiles; t += warps) {
-      for (int64_t f = F; f < F + L.tail_frames; ++f) {
-        const int64_t a0 = t * tile, a1 = min(n_sel, a0 + tile);
-        const double v = gather_item<3, RAW ? kFwdRaw : (W ? kFwdW : kFwdFit), kGatherDepth, true>(
-            L, L.coords + (size_t)f * L.n_atoms * 3, a0, a1, mean, lane);
-        if ((lane & 1) == 0) L.partial[((size_t)f * n_tiles + t) * kStatDoubles + (lane >> 1)] = v;
-      }
-      if (L.group_done && last_of_group(groups) && lane < L.tail_frames) finish_from_records(F + lane);
-      __syncwarp();
     }
+    if (lane < L.tail_frames) lane_finish(L, F + lane, tot, kMode);
+    return;
   }
-  if (gw >= nw || u0 >= u1) return;
 
-  auto unit_stages = [&](int64_t u) {
-    const int64_t t = u / groups;
-    return (int)((min(tile, n_sel - t * tile) + kLaneAtoms - 1) / kLaneAtoms);
-  };
-  // producer cursor (lane 0): unit pu, stage pk; n_issued stages so far
-  int64_t pu = u0;
-  int pk = 0, p_kst = unit_stages(u0);
+  const int64_t w0 = split.first(gw), w1 = split.first(gw + 1);
+  const int kst = split.stages;  // stages of a frame group
+  if (w0 >= w1) return;
+  // producer cursor (lane 0): stage pk of group pg; n_issued stages so far
+  const int64_t total = w1 - w0;
+  int64_t pg = w0 / kst;
+  int pk = (int)(w0 - pg * kst);
   int64_t n_issued = 0;
   // under the error-path test the first stage of CTA 0's warp 0 is never armed
   const bool withheld = L.wait.withhold && blockIdx.x == 0 && warp == 0;
   auto issue_next = [&]() {  // lane 0
-    const int64_t t = pu / groups, g = pu - t * groups;
     const int slot = (int)(n_issued % kLaneStages);
     unsigned char* dst = ring + slot * G::kStageBytes;
-    const int64_t a0 = t * tile + (int64_t)pk * kLaneAtoms;
+    const int64_t a0 = (int64_t)pk * kLaneAtoms;
     if (!(withheld && n_issued == 0)) {
       // the warp's earlier generic reads of this slot before the async writes
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -312,80 +365,78 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int64_t e = (int64_t)j * 3 * L.n_atoms + 3 * a0;
-          tma_load_2d(dst + j * QuadGeo::kBoxBytes, &map, (int)(e & ~int64_t(3)), (int)(g * 8), &full[slot]);
+          tma_load_2d(dst + j * QuadGeo::kBoxBytes, &map, (int)(e & ~int64_t(3)), (int)(pg * 8), &full[slot]);
         }
       } else {
 #pragma unroll
         for (int b = 0; b < LaneGeo<STRIDE>::kBoxes; ++b)
-          tma_load_2d(dst + b * 4096, &map, (int)(a0 * STRIDE + 32 * b), (int)(g * 32), &full[slot]);
+          tma_load_2d(dst + b * 4096, &map, (int)(a0 * STRIDE + 32 * b), (int)(pg * 32), &full[slot]);
       }
       bulk_copy_g2s(dst + G::kXBytes, L.lane_y + a0 * 3, G::kYBytes, &full[slot]);
       if (W) bulk_copy_g2s(dst + G::kXBytes + G::kYBytes, L.lane_w + a0, G::kWBytes, &full[slot]);
     }
     ++n_issued;
-    if (++pk == p_kst && ++pu < u1) {
+    if (++pk == kst) {
       pk = 0;
-      p_kst = unit_stages(pu);
+      ++pg;
     }
   };
   if (lane == 0)
-    while (n_issued < kLaneStages && pu < u1) issue_next();
+    while (n_issued < kLaneStages && n_issued < total) issue_next();
 
   // quad rows: this lane's float offset into its box row (stages start at
   // multiples of 32 atoms, so only the frame position matters)
   const int quad_off = QUAD ? (int)(((int64_t)(lane & 3) * 3 * L.n_atoms) & 3) : 0;
   int64_t n_done = 0;
   bool aborted = false;
-  for (int64_t u = u0; u < u1 && !aborted; ++u) {
-    const int64_t t = u / groups, g = u - t * groups;
-    const int kst = unit_stages(u);
-    double acc[15];
+  for (int64_t g = w0 / kst; g * kst < w1; ++g) {
+    // this warp's part of group g: stages [k0, k1)
+    const int k0 = (int)max((int64_t)0, w0 - g * kst), k1 = (int)min((int64_t)kst, w1 - g * kst);
+    double acc[15], tot[16];
 #pragma unroll
-    for (int e = 0; e < 15; ++e) acc[e] = 0.0;
-    for (int k = 0; k < kst; ++k) {
+    for (int e = 0; e < 15; ++e) acc[e] = tot[e] = 0.0;
+    tot[15] = 0.0;
+    for (int k = k0; k < k1; ++k) {
       const int slot = (int)(n_done % kLaneStages);
       const uint32_t parity = (uint32_t)((n_done / kLaneStages) & 1);
       if (!mbar_wait(&full[slot], parity, L.status, kStatusTimeoutFull, abort_flag, L.wait.limit_ns)) {
         aborted = true;
         break;
       }
-      const int64_t a0 = t * tile + (int64_t)k * kLaneAtoms;
-      const int valid = (int)min((int64_t)kLaneAtoms, n_sel - a0);
+      const int valid = (int)min((int64_t)kLaneAtoms, n_sel - (int64_t)k * kLaneAtoms);
       if (QUAD)
         stage_sums_quad<RAW, W>(acc, ring + slot * G::kStageBytes, lane, quad_off, valid, mean);
       else
         stage_sums<STRIDE, RAW, W>(acc, ring + slot * G::kStageBytes, lane, valid, mean);
       ++n_done;
       __syncwarp();
-      if (lane == 0 && pu < u1) issue_next();
+      if (lane == 0 && n_issued < total) issue_next();
+      // sums of kLaneBlock stages, then their sum: rounding grows with the longest chain
+      if ((k + 1) % kLaneBlock == 0 || k + 1 == k1) {
+#pragma unroll
+        for (int e = 0; e < 15; ++e) {
+          tot[e] += acc[e];
+          acc[e] = 0.0;
+        }
+      }
     }
     if (aborted) break;
     if (RAW) {  // the no-fit record holds sum |x - y|^2 in its first word
-      acc[0] += acc[1] + acc[2];
-      acc[1] = acc[2] = 0.0;
+      tot[0] += tot[1] + tot[2];
+      tot[1] = tot[2] = 0.0;
+    }
+    if (k1 - k0 < kst) {  // other warps hold the rest of the group
+      double* rec = split.record(L, gw, g) + lane;
+#pragma unroll
+      for (int e = 0; e < 15; ++e) __stcg(rec + e * 32, tot[e]);
+      if (!L.lane_fused) continue;
+      const int64_t wa = split.owner(g * kst), wb = split.owner((g + 1) * kst - 1);
+      if (!last_part(g, (int)(wb - wa) + 1)) continue;
+      split.add_records<4>(L, g, wa, wb + 1, 1, lane, tot);
     }
     const int64_t f = g * 32 + lane;
-    if (L.group_done && n_tiles == 1) {  // the unit is the frame
-      if (f < F) {
-        double tot[16];
-#pragma unroll
-        for (int e = 0; e < 15; ++e) tot[e] = acc[e];
-        tot[15] = 0.0;
-        finish_totals(L, f, tot, kMode);
-      }
-      __syncwarp();
-      continue;
-    }
-    if (f < F) {
-      double2* rec = reinterpret_cast<double2*>(L.partial + ((size_t)f * n_tiles + t) * kStatDoubles);
-#pragma unroll
-      for (int e = 0; e < 7; ++e) rec[e] = make_double2(acc[2 * e], acc[2 * e + 1]);
-      rec[7] = make_double2(acc[14], 0.0);
-    }
-    if (L.group_done) {
-      if (last_of_group(g) && f < F) finish_from_records(f);
-      __syncwarp();
-    }
+    if (f < F) lane_finish(L, f, tot, kMode);
+    __syncwarp();
   }
 
   // after an abort, copies this warp issued may still be landing (a withheld
@@ -394,6 +445,39 @@ __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __gri
     for (int64_t j = n_done; j < n_issued; ++j)
       if (!(withheld && j == 0)) mbar_drain(&full[j % kLaneStages], (uint32_t)((j / kLaneStages) & 1), L.status);
   }
+}
+
+// Frame groups spread over more warps than one of them should add up: a CTA per
+// group, its warps adding every kFinalizeWarps-th record, then a lane per frame.
+constexpr int kFinalizeWarps = 16;
+
+template <int MODE>
+__global__ void __launch_bounds__(kFinalizeWarps * 32) lanes_finalize_kernel(const FrameLaunch L) {
+  extern __shared__ double red[];  // [kFinalizeWarps][15][32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const LaneSplit split(L);
+  const int64_t g = blockIdx.x;
+  const int64_t wa = split.owner(g * split.stages), wb = split.owner((g + 1) * split.stages - 1);
+  if (wa == wb) return;  // one warp had the whole group
+  double tot[16];
+  split.add_records<4>(L, g, wa + warp, wb + 1, kFinalizeWarps, lane, tot);
+#pragma unroll
+  for (int e = 0; e < 15; ++e) red[(warp * 15 + e) * 32 + lane] = tot[e];
+  __syncthreads();
+  // element e of every frame by warp e
+  if (warp < 15) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < kFinalizeWarps; ++w) s += red[(w * 15 + warp) * 32 + lane];
+    red[warp * 32 + lane] = s;  // slot (0, e): read by this warp alone
+  }
+  __syncthreads();
+  const int64_t f = g * 32 + lane;
+  if (warp != 0 || f >= L.n_frames) return;
+#pragma unroll
+  for (int e = 0; e < 15; ++e) tot[e] = red[e * 32 + lane];
+  tot[15] = 0.0;
+  lane_finish(L, f, tot, MODE);
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -412,10 +496,6 @@ EncodeTiled encode_fn() {
   }
   fn = reinterpret_cast<EncodeTiled>(p);
   return fn;
-}
-
-int64_t lane_units(const FrameLaunch& L, int64_t tile) {
-  return ((L.n_frames + 31) / 32) * ((L.lane_atoms + tile - 1) / tile);
 }
 
 template <int STRIDE, bool RAW, bool QUAD = false>
@@ -465,7 +545,18 @@ cudaError_t launch_lanes(const FrameLaunch& L, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
-  kern<<<L.grid, kLaneWarps * 32, G::kSmemBytes, s>>>(map, L);
+  const int grid = (L.lane_warps + L.lane_tail_warps + kLaneWarps - 1) / kLaneWarps;
+  kern<<<grid, kLaneWarps * 32, G::kSmemBytes, s>>>(map, L);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || L.lane_fused) return e;
+  auto fin = lanes_finalize_kernel<RAW ? kFwdRaw : kFwdFit>;
+  constexpr int kFinBytes = kFinalizeWarps * 15 * 32 * 8;
+  static bool fin_done[64] = {};
+  if (!fin_done[dev]) {
+    if ((e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinBytes)) != cudaSuccess) return e;
+    fin_done[dev] = true;
+  }
+  fin<<<(unsigned)((L.n_frames + 31) / 32), kFinalizeWarps * 32, kFinBytes, s>>>(L);
   return cudaGetLastError();
 }
 
@@ -530,65 +621,67 @@ static int lanes_slots(const FrameLaunch& L, int sm_count) {
   return sm_count * o * kLaneWarps;
 }
 
-// Active warps for `slots` warp slots: every warp gets the same number of
-// whole units (the last one possibly fewer).
-static int64_t lane_warps(const FrameLaunch& L, int64_t slots) {
-  const int64_t units = lane_units(L, L.tile_atoms);
-  const int64_t per = (units + slots - 1) / slots;
-  return std::max<int64_t>(1, (units + per - 1) / per);
-}
-
+// Against the atom-major kernel, whose cost is its (1,024-atom tile, frame) items
+// and its finalize launch (us, lanes / atom-major): 8,000 x 128 15.5 / 39; 4,000 x 500
+// 18.4 / 26.6; 1,500 x 2,000 23.3 / 24.7; 5,001 x 3,001 50 / 59; 600 x 4,000 22.7 / 21.5;
+// 2,400 x 1,000 21.6 / 20.9.  Few groups leave lanes empty and many parts to add:
+// 256 x 40,000 41.9 / 44.1, but 160 x 20,000 29.3 / 25.0, 64 x 400,000 102 / 94.
+// With weights it is ahead at every size measured (300 x 100,000, superposition
+// with masses: 211 / 265; 2,000 x 2,000 47 / 49); an expanded selection's
+// alternative is the gathered kernel.
 bool lanes_worthwhile(const FrameLaunch& L, int sm_count) {
-  // fewer (256-atom tile, 32-frame group) units than two per SM: the
-  // atom-major kernel's (tile, frame) items spread better
-  return lane_units(L, 256) >= 2 * (int64_t)sm_count;
+  const int64_t groups = (L.n_frames + 31) / 32;
+  if (L.lane_w) return groups * ((L.lane_atoms + 255) / 256) >= 2 * (int64_t)sm_count;
+  return groups >= 8 && L.n_frames * ((L.lane_atoms + 1023) / 1024) >= 20 * (int64_t)sm_count;
 }
 
-int lanes_tile(const FrameLaunch& L, int sm_count) {
-  // Tile size, any multiple of 32 from 128 to 2,048 atoms, minimising the
-  // busiest warp's bytes: (units per warp) x (tile bytes + its 128-byte partial,
-  // written and read back).  Large tiles mean few records; small ones balance
-  // short runs (few frames or few atoms) over all warp slots.  5,001 frames x
-  // 3,001 atoms: 448 atoms (1,099 units on 1,184 slots) instead of 512 (942).
-  const int64_t slots = lanes_slots(L, sm_count);
-  int64_t best = kLaneTile, best_cost = -1;
-  for (int64_t tile = kLaneTile; tile >= 128; tile -= kLaneAtoms) {
-    const int64_t per = (lane_units(L, tile) + slots - 1) / slots;
-    const int64_t cost = per * (tile * L.stride * 4 + 256);
-    if (best_cost < 0 || cost < best_cost) {
-      best = tile;
-      best_cost = cost;
-    }
+int lanes_grid(const FrameLaunch& L, int sm_count) { return lanes_slots(L, sm_count) / kLaneWarps; }
+
+// Two records per warp and the tail frames' tiles.
+size_t lane_record_bytes(const FrameLaunch& L, int sm_count) {
+  return (size_t)lanes_slots(L, sm_count) * (2 * 16 * 32 + 3 * 16) * sizeof(double);
+}
+
+// Splits L's frames over `slots` warps.
+static void lanes_split(FrameLaunch& L, int64_t slots) {
+  if (L.tail_frames > 0) {
+    // warps for the tail frames by their share of the work (a warp streams ~16 times
+    // as many atom-frames across lanes as it gathers along one frame)
+    const int64_t part = 16 * L.tail_frames;
+    const int64_t d = std::min(std::max<int64_t>(1, slots / 2 / L.tail_frames),
+                               (slots * 16 + L.n_frames + part - 1) / (L.n_frames + part));  // per frame
+    L.lane_tail_tile = ((L.lane_atoms + d - 1) / d + 127) / 128 * 128;
+    L.lane_tail_warps = (int)(L.tail_frames * ((L.lane_atoms + L.lane_tail_tile - 1) / L.lane_tail_tile));
+    slots -= L.lane_tail_warps;
   }
-  return (int)best;
-}
-
-int lanes_grid(const FrameLaunch& L, int sm_count) {
-  return (int)((lane_warps(L, lanes_slots(L, sm_count)) + kLaneWarps - 1) / kLaneWarps);
+  const int64_t groups = (L.n_frames + 31) / 32, stages = (L.lane_atoms + kLaneAtoms - 1) / kLaneAtoms;
+  const int64_t total = groups * stages;
+  int64_t nw = std::max<int64_t>(1, std::min(slots, total / kLaneMinStages));
+  // whole groups where that costs the busiest warp only a few stages
+  const int64_t runs = std::min(groups, nw);
+  const int64_t longest = (groups + runs - 1) / runs * stages;
+  L.lane_whole = longest <= (total + nw - 1) / nw + kLaneWholeStages;
+  if (L.lane_whole) nw = runs;
+  L.lane_warps = (int)nw;
+  L.lane_fused = L.lane_whole || (nw + groups - 1) / groups + 1 <= kLaneFinishParts;
 }
 
 cudaError_t launch_lanes_forward(const FrameLaunch& L, bool raw, cudaStream_t s) {
   FrameLaunch K = L;
-  const bool w = L.lane_w != nullptr;
-  if (lanes_quad(L)) {
-    // whole quad rows, and the last n_frames mod 4 frames with plain loads
-    const int64_t main = L.n_frames & ~int64_t(3);
-    if (main > 0) {  // a batch of fewer than 4 frames has no quad row
-      K.n_frames = main;
-      K.tail_frames = (int)(L.n_frames - main);
-      K.lane_warps = (int)lane_warps(K, (int64_t)L.grid * kLaneWarps);
-      cudaError_t e = w ? (raw ? launch_lanes<3, true, true, true>(K, s) : launch_lanes<3, false, true, true>(K, s))
-                        : (raw ? launch_lanes<3, true, false, true>(K, s) : launch_lanes<3, false, false, true>(K, s));
-      return e;
-    }
-    static int sms[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    return launch_gather_partials(L, raw, sms[dev], s);
+  const bool w = L.lane_w != nullptr, quad = lanes_quad(L);
+  if (quad) {  // whole quad rows, and the last n_frames mod 4 frames with plain loads
+    K.n_frames = L.n_frames & ~int64_t(3);
+    K.tail_frames = (int)(L.n_frames - K.n_frames);
   }
-  K.lane_warps = (int)lane_warps(L, (int64_t)L.grid * kLaneWarps);
+  lanes_split(K, std::max<int64_t>(2, (int64_t)L.grid * kLaneWarps));
+  cudaError_t e = cudaSuccess;
+  if (!L.done_cleared && ((K.lane_fused && !K.lane_whole) || K.tail_frames > 0)) {
+    e = cudaMemsetAsync(K.group_done, 0, (size_t)frame_groups(K.n_frames) * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+  }
+  if (quad)
+    return w ? (raw ? launch_lanes<3, true, true, true>(K, s) : launch_lanes<3, false, true, true>(K, s))
+             : (raw ? launch_lanes<3, true, false, true>(K, s) : launch_lanes<3, false, false, true>(K, s));
   if (L.stride == 4) {
     if (w) return raw ? launch_lanes<4, true, true>(K, s) : launch_lanes<4, false, true>(K, s);
     return raw ? launch_lanes<4, true, false>(K, s) : launch_lanes<4, false, false>(K, s);

@@ -403,7 +403,24 @@ int64_t frame_batch(size_t fit, int64_t n_frames) {
 // (same tiles, same partials).  The frames-across-lanes kernel needs no check:
 // it only runs when the frame stride is a multiple of 16 bytes.
 void keep_aligned(wmd::FrameLaunch& B) {
+  if (B.lanes && B.n_frames < 4 && B.stride == 3 && (B.n_atoms & 3) != 0) {  // no quad row: gathered, 1,024-atom tiles
+    B.lanes = false;
+    B.gather = true;
+  }
   if (!B.lanes && !B.gather && (reinterpret_cast<uintptr_t>(B.coords) & 15u) != 0) B.gather = true;
+}
+
+// Scratch of a batch of L's frames: per-frame sums (totals: of a lanes launch too), and
+// the lanes kernel's records behind them.
+struct FrameScratch {
+  size_t per_frame, fixed;
+};
+FrameScratch frame_scratch(wmd_ctx* ctx, const wmd::FrameLaunch& L, bool totals) {
+  const size_t rec = wmd::kStatDoubles * sizeof(double);
+  if (!L.lanes) return {(size_t)std::max(wmd::frame_tiles(L), 1) * rec, 0};
+  // a last batch of up to 3 frames may run the gathered kernel
+  const size_t rest = (size_t)(3 * ((L.ref.n_sel + L.tile_atoms - 1) / L.tile_atoms)) * rec;
+  return {totals ? rec : 0, rest + wmd::lane_record_bytes(L, ctx->sm_count)};
 }
 
 // Runs the forward over device-resident frames, splitting into frame batches
@@ -418,11 +435,11 @@ int forward_device(wmd_ctx* ctx, const float* dcoords, int64_t n_frames, int64_t
   L.n_frames = n_frames;
   apply_lanes(ctx, L, dsel);
   wmd::frame_plan(L, ctx->sm_count);
-  const int tiles = wmd::frame_tiles(L);
-  const size_t per_frame = (size_t)tiles * wmd::kStatDoubles * sizeof(double);
-  const int64_t batch = frame_batch(kPartialBytesMax / per_frame, n_frames);
+  const FrameScratch fs = frame_scratch(ctx, L, false);
+  const int64_t batch =
+      frame_batch(kPartialBytesMax / std::max(fs.per_frame, wmd::kStatDoubles * sizeof(double)), n_frames);
   {
-    int rc = ensure(ctx, ctx->partial, per_frame * (size_t)batch);
+    int rc = ensure(ctx, ctx->partial, fs.per_frame * (size_t)batch + fs.fixed);
     if (rc) return rc;
   }
   if (align) {
@@ -441,14 +458,14 @@ int forward_device(wmd_ctx* ctx, const float* dcoords, int64_t n_frames, int64_t
     }
     B.group_done = counts + 1;
     B.coords = dcoords + (size_t)f0 * n_atoms * stride;
-    keep_aligned(B);
     B.n_frames = nf;
+    keep_aligned(B);
     B.out.rmsd = o.rmsd ? o.rmsd + f0 : nullptr;
     B.out.stats = o.stats ? o.stats + f0 * wmd::kStatDoubles : nullptr;
     B.out.cov = o.cov ? o.cov + f0 * 9 : nullptr;
     B.out.sum_x2 = o.sum_x2 ? o.sum_x2 + f0 : nullptr;
     B.out.sum_y2 = o.sum_y2 ? o.sum_y2 + f0 : nullptr;
-    B.partial = static_cast<double*>(ctx->partial.ptr);
+    B.partial = B.lane_rec = static_cast<double*>(ctx->partial.ptr);
     B.grid = wmd::frame_grid(B, ctx->sm_count, false);
     CU(wmd::launch_rmsd_forward(B, s), "rmsd forward launch");
   }
@@ -901,20 +918,23 @@ static int superpose_device(wmd_ctx* ctx, const float* dcoords, int64_t n_frames
   L.n_frames = n_frames;
   apply_lanes(ctx, L, dsel);
   wmd::frame_plan(L, ctx->sm_count);
-  const int tiles = wmd::frame_tiles(L);
-  const size_t per_frame = (size_t)std::max(tiles, 1) * wmd::kStatDoubles * sizeof(double);
-  const int64_t batch = frame_batch(kPartialBytesMax / per_frame, n_frames);
+  L.lane_totals = true;
+  const FrameScratch fs = frame_scratch(ctx, L, true);
+  const int64_t batch = frame_batch(kPartialBytesMax / fs.per_frame, n_frames);
   int rc;
-  if ((rc = ensure(ctx, ctx->partial, per_frame * (size_t)batch)) ||
+  if ((rc = ensure(ctx, ctx->partial, fs.per_frame * (size_t)batch + fs.fixed)) ||
+      (rc = ensure(ctx, ctx->refine_count, (size_t)(1 + wmd::frame_groups(batch)) * sizeof(unsigned), true)) ||
       (rc = ensure(ctx, ctx->rot, (size_t)batch * wmd::kStatDoubles * sizeof(double))))
     return rc;
   for (int64_t f0 = 0; f0 < n_frames; f0 += batch) {
     const int64_t nf = std::min(batch, n_frames - f0);
     wmd::FrameLaunch B = L;
     B.coords = dcoords + (size_t)f0 * n_atoms * stride;
-    keep_aligned(B);
     B.n_frames = nf;
-    B.partial = static_cast<double*>(ctx->partial.ptr);
+    keep_aligned(B);
+    B.lane_rec = static_cast<double*>(ctx->partial.ptr);  // the records first, they are a multiple of 256 bytes
+    B.partial = B.lanes ? B.lane_rec + wmd::lane_record_bytes(B, ctx->sm_count) / sizeof(double) : B.lane_rec;
+    B.group_done = static_cast<unsigned*>(ctx->refine_count.ptr) + 1;
     B.grid = wmd::frame_grid(B, ctx->sm_count, false);
     if (ref->info.n_sel > 0) {
       if (ref->info.w) CU(wmd::launch_rmsd_stream_weighted(B, s), "superpose statistics");

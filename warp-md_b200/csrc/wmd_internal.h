@@ -56,10 +56,17 @@ struct FrameLaunch {
   int stride = 3;                 // floats per atom (3 or 4)
   const uint32_t* sel = nullptr;  // device indices, or null (dense 0..n_sel-1)
   bool gather = false;            // plain loads (selection or unaligned base)
-  int tile_atoms = 2048;          // atoms per tile (kConsumerThreads * atoms/thread, or kLaneTile)
+  int tile_atoms = 2048;          // atoms per tile (kConsumerThreads * atoms/thread, or gather_tile)
   bool lanes = false;             // frames-across-lanes forward kernel (rmsd_lanes.cu)
-  int lane_warps = 0;             // its active warps (set at launch)
-  int tail_frames = 0;            // its frames past n_frames that fill no quad row (set at launch)
+  // set at launch: its active warps; runs of whole frame groups; groups finished by
+  // the last of their warps (else by a second kernel); the frames past n_frames
+  // that fill no quad row, with warps of their own and their tile of atoms
+  int lane_warps = 0;
+  bool lane_whole = false;
+  bool lane_fused = false;
+  int tail_frames = 0;
+  int lane_tail_warps = 0;
+  int64_t lane_tail_tile = 0;
   int64_t lane_atom0 = 0;         // its atoms: [lane_atom0, lane_atom0 + lane_atoms) of every frame
   int64_t lane_atoms = 0;
   const double* lane_y = nullptr; // reference values over those atoms (centred, weighted), +32 zero atoms
@@ -71,11 +78,13 @@ struct FrameLaunch {
   const double* rot = nullptr;  // [n_frames][16] from the backward prologue
   float* grad = nullptr;        // [n_frames][n_atoms][3]
   // scratch
-  double* partial = nullptr;    // [n_frames][n_tiles][16] per-tile sums
+  double* partial = nullptr;    // [n_frames][n_tiles][16] per-tile sums (lanes with lane_totals: [n_frames][16])
+  double* lane_rec = nullptr;   // lanes: lane_record_bytes of scratch
+  bool lane_totals = false;     // lanes: leave the frames' sums in partial instead of finishing them
   double* refine = nullptr;     // [n_frames][16] records of frames needing the residual pass
   unsigned* refine_count = nullptr;  // number of records, zeroed before each forward
-  unsigned* group_done = nullptr;    // [frame_groups] tiles stored per 32-frame group, follows *refine_count
-                                     // (cleared with it), or null: rmsd_finalize_kernel finishes the frames
+  unsigned* group_done = nullptr;    // lanes: [frame_groups] parts stored per 32-frame group and of the tail
+  bool done_cleared = false;         // group_done is zero already (it follows *refine_count, cleared with it)
   int* status = nullptr;        // device-visible status word (mapped host)
   WaitCfg wait;                 // limits of the bounded waits
   int grid = 0;                 // CTAs (persistent)
@@ -93,13 +102,11 @@ int frame_tiles(const FrameLaunch& L);
 // Picks the forward kernel for a launch (sets lanes and tile_atoms); call
 // before sizing the partials with frame_tiles.
 void frame_plan(FrameLaunch& L, int sm_count);
-// frames-across-lanes forward (rmsd_lanes.cu): at most 2,048 atoms per
-// partial record
-constexpr int kLaneTile = 2048;
+// frames-across-lanes forward (rmsd_lanes.cu)
 bool lanes_eligible(const FrameLaunch& L);
 bool lanes_worthwhile(const FrameLaunch& L, int sm_count);
-int lanes_tile(const FrameLaunch& L, int sm_count);
 int lanes_grid(const FrameLaunch& L, int sm_count);
+size_t lane_record_bytes(const FrameLaunch& L, int sm_count);
 cudaError_t launch_lanes_forward(const FrameLaunch& L, bool raw, cudaStream_t s);
 // Expands a strictly increasing device selection's reference values (yc
 // [n_sel][3]) and weights (w, or all 1 when null) onto the atom span starting
@@ -109,8 +116,6 @@ cudaError_t launch_lanes_expand(const uint32_t* sel, int64_t n_sel, int64_t a0, 
 size_t frame_smem_bytes(int stride, int tile_atoms);
 // Entries of FrameLaunch::group_done: the 32-frame groups and the tail.
 inline int64_t frame_groups(int64_t n_frames) { return (n_frames + 31) / 32 + 1; }
-// Most tiles a lane adds up itself (rmsd_lanes.cu)
-constexpr int kLaneFinishTiles = 16;
 // Forward: zeroes L.refine_count, runs the fused kernel, then the residual pass
 // over the frames it flagged.
 cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s);
@@ -131,11 +136,6 @@ cudaError_t launch_rmsd_backward(const FrameLaunch& L, const double* stats, cons
                                  const double* grad_f64, int64_t grad_stride, double* rot_scratch, cudaStream_t s);
 // occupancy-derived persistent grid for a launch
 int frame_grid(const FrameLaunch& L, int sm_count, bool backward);
-// The gathered kernel's (tile, frame) partials for L's frames with tiles of
-// L.tile_atoms over a dense selection: the frames-across-lanes kernel's layout,
-// for frames it leaves to others (raw: the no-fit record).
-cudaError_t launch_gather_partials(const FrameLaunch& L, bool raw, int sm_count, cudaStream_t s);
-
 // Whole-frame kernels for many frames of up to kVgMaxAtoms atoms
 // (rmsd_vg.cu): forward (rmsd and the 16-double records of
 // wmd_rmsd_forward), backward (gradient from those records) and both in one
