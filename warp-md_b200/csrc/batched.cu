@@ -297,8 +297,11 @@ __global__ void __launch_bounds__(kThreads, 4) batched_stream_kernel(const Batch
 
 // One CTA per trajectory: y_c = y - mean(y) into the workspace, and the
 // statistics the finisher needs (sum of y_c, G_y), in fixed-order trees.
-__global__ void __launch_bounds__(256) batched_ref_prep(BatchSeg* segs) {
-  __shared__ double red[8][3];
+// Bound by the latency of its three passes (19,468 atoms: 256 threads 43 us, 1,024 37 us).
+constexpr int kPrepThreads = 1024;
+
+__global__ void __launch_bounds__(kPrepThreads) batched_ref_prep(BatchSeg* segs) {
+  __shared__ double red[kPrepThreads / 32][3];
   __shared__ double bc[3];
   BatchSeg& s = segs[blockIdx.x];
   const float* ref = s.ref;
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(256) batched_ref_prep(BatchSeg* segs) {
     __syncthreads();
     if (tid == 0) {
       double s0 = 0, s1 = 0, s2 = 0;
-      for (int w = 0; w < 8; ++w) { s0 += red[w][0]; s1 += red[w][1]; s2 += red[w][2]; }
+      for (int w = 0; w < kPrepThreads / 32; ++w) { s0 += red[w][0]; s1 += red[w][1]; s2 += red[w][2]; }
       bc[0] = s0; bc[1] = s1; bc[2] = s2;
     }
     __syncthreads();
@@ -329,12 +332,14 @@ __global__ void __launch_bounds__(256) batched_ref_prep(BatchSeg* segs) {
   }
   if (s.n_frames == 0) return;
   double m0 = 0, m1 = 0, m2 = 0;
+#pragma unroll 4
   for (int64_t k = tid; k < n; k += blockDim.x) { m0 += ref[k * 3]; m1 += ref[k * 3 + 1]; m2 += ref[k * 3 + 2]; }
   sum3(m0, m1, m2);
   const double inv = 1.0 / (double)n;
   m0 *= inv; m1 *= inv; m2 *= inv;
   if (tid == 0) { s.mean_y[0] = m0; s.mean_y[1] = m1; s.mean_y[2] = m2; }
   double c0 = 0, c1 = 0, c2 = 0;
+#pragma unroll 4
   for (int64_t k = tid; k < n; k += blockDim.x) {
     const double a = (double)ref[k * 3] - m0, b = (double)ref[k * 3 + 1] - m1, c = (double)ref[k * 3 + 2] - m2;
     yc[k * 3] = a; yc[k * 3 + 1] = b; yc[k * 3 + 2] = c;
@@ -342,6 +347,7 @@ __global__ void __launch_bounds__(256) batched_ref_prep(BatchSeg* segs) {
   }
   sum3(c0, c1, c2);
   double g0 = 0, g1 = 0, g2 = 0;
+#pragma unroll 4
   for (int64_t k = tid; k < n; k += blockDim.x) {
     const double a = yc[k * 3] - c0 * inv, b = yc[k * 3 + 1] - c1 * inv, c = yc[k * 3 + 2] - c2 * inv;
     g0 += a * a; g1 += b * b; g2 += c * c;
@@ -355,25 +361,43 @@ __global__ void __launch_bounds__(256) batched_ref_prep(BatchSeg* segs) {
 
 // Frames of the batch, a lane each: the warp first sums the tile partials of
 // its 32 frames in tile order (two frames at a time, 16 lanes per frame, into
-// shared memory), then every lane runs QCP for its own frame -- the FP64
+// shared memory, all in flight where the 32 frames belong to one trajectory:
+// 82,000 frames 55 -> 49 us, the rest is QCP and the rotation), then every lane runs QCP for its own frame -- the FP64
 // Newton iteration and, with gradients, the rotation from the eigenvector --
 // so the warp issues each instruction once for 32 frames.
-__global__ void __launch_bounds__(256) batched_finalize(const BatchLaunch B) {
-  __shared__ double st[8][32][17];
+constexpr int kFinWarps = 2;  // few frames: warps on more SMs
+
+__global__ void __launch_bounds__(kFinWarps * 32) batched_finalize(const BatchLaunch B) {
+  __shared__ double st[kFinWarps][32][17];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t base = ((int64_t)blockIdx.x * 8 + warp) * 32;
+  const int64_t base = ((int64_t)blockIdx.x * kFinWarps + warp) * 32;
   if (base >= B.total_frames) return;
-  for (int i = 0; i < 16; ++i) {
-    const int fl = 2 * i + (lane >> 4);
-    const int64_t g = base + fl;
-    double v = 0.0;
-    if (g < B.total_frames) {
-      const BatchSeg& sg = B.segs[seg_of(B.segs, B.n_segs, g, true)];
-      const int64_t f = g - sg.frame0;
-      for (int t = 0; t < sg.n_tiles; ++t)
-        v += B.partial[(size_t)(sg.item0 + (int64_t)t * sg.n_frames + f) * kStatDoubles + (lane & 15)];
+  const BatchSeg& s0 = B.segs[seg_of(B.segs, B.n_segs, base, true)];
+  if (base + 32 <= s0.frame0 + s0.n_frames) {
+    // all 32 frames of one trajectory: 16 records in flight per lane
+    const size_t tile = (size_t)s0.n_frames * kStatDoubles;
+    const double* part = B.partial + (size_t)(s0.item0 + base - s0.frame0 + (lane >> 4)) * kStatDoubles + (lane & 15);
+    double v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = 0.0;
+    for (int t = 0; t < s0.n_tiles; ++t, part += tile)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] += part[2 * i * kStatDoubles];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) st[warp][2 * i + (lane >> 4)][lane & 15] = v[i];
+  } else {
+    for (int i = 0; i < 16; ++i) {
+      const int fl = 2 * i + (lane >> 4);
+      const int64_t g = base + fl;
+      double v = 0.0;
+      if (g < B.total_frames) {
+        const BatchSeg& sg = B.segs[seg_of(B.segs, B.n_segs, g, true)];
+        const int64_t f = g - sg.frame0;
+        for (int t = 0; t < sg.n_tiles; ++t)
+          v += B.partial[(size_t)(sg.item0 + (int64_t)t * sg.n_frames + f) * kStatDoubles + (lane & 15)];
+      }
+      st[warp][fl][lane & 15] = v;
     }
-    st[warp][fl][lane & 15] = v;
   }
   __syncwarp();
   const int64_t g = base + lane;
@@ -845,11 +869,17 @@ __global__ void __launch_bounds__(kThreads, 4) batched_frame_kernel(const BatchL
 //   quad rows (tma = 2): 4 boxes of [8 quad rows x 100 floats], box j holding
 //       frame position j of quad rows 8g .. 8g + 7 from the 16-byte boundary
 //       at or below the stage's first atom; lane 4i + j reads row i of box j
-//       at a fixed float offset.  Lanes of the last n_frames mod 4 frames
-//       (past the last whole quad row) read their atoms with plain loads.
-// Without a map (tma = 0) every lane bulk-copies its own frame's row, the
-// 16-byte hull of 32 atoms (at most 400 bytes).  Warps take contiguous runs
-// of units of equal estimated cost.
+//       at a fixed float offset.
+// Without a map (tma = 0), and in the group that holds the last n_frames mod 4
+// frames (no whole quad row), every lane bulk-copies its own frame's row, the
+// 16-byte hull of 32 atoms (at most 400 bytes).
+// Warps take equal runs of stages.  A run that begins inside a unit leaves that
+// part's sums in the warp's extra record, which batched_lanes_fold adds to the
+// unit's.  With runs of whole units of equal estimated cost (7 units a warp) the longest
+// run was 12 % above the mean, and the tail frames' plain loads stretched their
+// warps' runs.  Measured: 277 million atom-frames in 30 trajectories 671 -> 604 + 7 us;
+// two of 20,000 frames x 1,024 atoms 160 -> 97 us.  HBM alone: 509 us (5.5 of 6.5
+// TB/s; FP64 and issue slots are each below half busy at two warps a scheduler).
 // ---------------------------------------------------------------------------
 constexpr int kBLWarps = 4;
 constexpr int kBLStages = 2;
@@ -872,12 +902,12 @@ __device__ __forceinline__ void bl_tma_load_2d(void* dst, const CUtensorMap* map
       : "memory");
 }
 
-// last segment whose units start at or before cost c
+// last segment whose stages start at or before stage c
 __device__ __forceinline__ int lane_seg_of(const BatchSeg* segs, int n, int64_t c) {
   int lo = 0, hi = n - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (segs[mid].lane_cost0 <= c) lo = mid;
+    if (segs[mid].lane_stage0 <= c) lo = mid;
     else hi = mid - 1;
   }
   return lo;
@@ -888,13 +918,29 @@ struct LaneCur {
   int64_t k;  // unit within the segment
 };
 
+// the unit that holds stage c, and the stage's index in it
+__device__ __forceinline__ LaneCur lane_unit_of(const BatchLaunch& B, int64_t c, int& j) {
+  LaneCur u;
+  u.seg = lane_seg_of(B.segs, B.n_segs, c);
+  const BatchSeg& S = B.segs[u.seg];
+  const int64_t off = c - S.lane_stage0, full = S.lane_full_units * S.lane_unit_stages;
+  if (off < full) {
+    u.k = off / S.lane_unit_stages;
+    j = (int)(off - u.k * S.lane_unit_stages);
+  } else {
+    u.k = (off - full) / S.lane_last_stages;
+    j = (int)(off - full - u.k * S.lane_last_stages);
+    u.k += S.lane_full_units;
+  }
+  return u;
+}
+
 // The fields of a trajectory the lanes kernel reads per stage and per unit,
 // held in registers while a cursor stays in that trajectory.
 struct LaneSeg {
   const float* coords;
   const double* yc;
   int64_t n_atoms, n_frames, groups, item0;
-  int64_t cost0, full_units, unit_cost, last_cost;
   int tma;
 };
 
@@ -906,17 +952,8 @@ __device__ __forceinline__ LaneSeg lane_seg(const BatchSeg& S) {
   v.n_frames = S.n_frames;
   v.groups = (S.n_frames + 31) / 32;
   v.item0 = S.item0;
-  v.cost0 = S.lane_cost0;
-  v.full_units = S.lane_full_units;
-  v.unit_cost = S.lane_unit_cost;
-  v.last_cost = S.lane_last_cost;
   v.tma = S.tma;
   return v;
-}
-
-// a unit's starting cost: whole-tile units first, then the last tile's
-__device__ __forceinline__ int64_t lane_unit_start(const LaneSeg& v, int64_t k) {
-  return v.cost0 + (k <= v.full_units ? k * v.unit_cost : v.full_units * v.unit_cost + (k - v.full_units) * v.last_cost);
 }
 
 __device__ __forceinline__ void lane_skip_empty(const BatchLaunch& B, LaneCur& c) {
@@ -943,30 +980,17 @@ __global__ void __launch_bounds__(kBLWarps * 32) batched_lanes_kernel(const Batc
     fence_barrier_init();
   }
   __syncthreads();
-  const int64_t nw = (int64_t)gridDim.x * kBLWarps, gw = (int64_t)blockIdx.x * kBLWarps + warp;
-  const int64_t C0 = B.total_lane_cost * gw / nw, C1 = B.total_lane_cost * (gw + 1) / nw;
-  if (C0 >= C1 || B.n_segs == 0) return;
-  // first unit starting at or after C0
-  LaneCur first;
-  first.seg = lane_seg_of(B.segs, B.n_segs, C0);
-  {
-    const BatchSeg& S = B.segs[first.seg];
-    const int64_t off = C0 - S.lane_cost0;
-    const int64_t full = S.lane_full_units * S.lane_unit_cost;
-    if (S.lane_units <= 0) first.k = 0;
-    else if (off <= full) first.k = (off + S.lane_unit_cost - 1) / S.lane_unit_cost;
-    else first.k = S.lane_full_units + (off - full + S.lane_last_cost - 1) / S.lane_last_cost;
-  }
-  lane_skip_empty(B, first);
+  const int64_t nw = B.lane_warps, gw = (int64_t)blockIdx.x * kBLWarps + warp;
+  if (gw >= nw) return;
+  const int64_t C0 = B.total_lane_stages * gw / nw, C1 = B.total_lane_stages * (gw + 1) / nw;
+  int first_j = 0;
+  const LaneCur first = lane_unit_of(B, C0, first_j);
   // a cursor's trajectory view, reloaded when the cursor enters another trajectory
   auto view = [&](const LaneCur& c, int& vseg, LaneSeg& v) {
     if (c.seg < B.n_segs && c.seg != vseg) {
       v = lane_seg(B.segs[c.seg]);
       vseg = c.seg;
     }
-  };
-  auto starts_before_end = [&](const LaneCur& c, const LaneSeg& v) {
-    return c.seg < B.n_segs && lane_unit_start(v, c.k) < C1;
   };
   auto unit_stages = [&](const LaneCur& c, const LaneSeg& v) {
     const int64_t t = c.k / v.groups;
@@ -977,11 +1001,15 @@ __global__ void __launch_bounds__(kBLWarps * 32) batched_lanes_kernel(const Batc
   int pv_seg = -1;
   LaneSeg pv;
   view(pc, pv_seg, pv);
-  int pj = 0;
-  bool p_live = starts_before_end(pc, pv);
-  int p_st = p_live ? unit_stages(pc, pv) : 0;
-  int64_t pt = p_live ? pc.k / pv.groups : 0, pg = p_live ? pc.k - pt * pv.groups : 0;
+  int pj = first_j;
+  int p_st = unit_stages(pc, pv);
+  int64_t pt = pc.k / pv.groups, pg = pc.k - pt * pv.groups;
   int64_t n_issued = 0;
+  const int64_t total = C1 - C0;
+  auto unit_tma = [&](const LaneSeg& v, int64_t g) {
+    return v.tma == 2 && g == v.groups - 1 && (v.n_frames & 3) != 0 ? 0 : v.tma;
+  };
+  int p_tma = unit_tma(pv, pg);
   auto issue_next = [&]() {
     const int64_t t = pt, g = pg;
     const int64_t a0 = t * T + (int64_t)pj * 32;
@@ -992,11 +1020,11 @@ __global__ void __launch_bounds__(kBLWarps * 32) batched_lanes_kernel(const Batc
     unsigned char* dst = st + lane * kBLRow;
     const int64_t f = g * 32 + lane;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (pv.tma) {
+    if (p_tma) {
       if (lane == 0) {
         const CUtensorMap* map = B.maps + pc.seg;
-        mbar_arrive_expect_tx(&full[slot], (pv.tma == 1 ? 3 * 4096 : 4 * kBLQuadBox) + kBLYBytes);
-        if (pv.tma == 1) {
+        mbar_arrive_expect_tx(&full[slot], (p_tma == 1 ? 3 * 4096 : 4 * kBLQuadBox) + kBLYBytes);
+        if (p_tma == 1) {
 #pragma unroll
           for (int b = 0; b < 3; ++b) bl_tma_load_2d(st + b * 4096, map, (int)(a0 * 3 + 32 * b), (int)(g * 32), &full[slot]);
         } else {
@@ -1035,22 +1063,18 @@ __global__ void __launch_bounds__(kBLWarps * 32) batched_lanes_kernel(const Batc
       if (lane == 0) bulk_copy_g2s(ys, pv.yc + a0 * 3, kBLYBytes, &full[slot]);
     }
     ++n_issued;
-    if (++pj == p_st) {
+    if (++pj == p_st && n_issued < total) {
       pj = 0;
       ++pc.k;
       lane_skip_empty(B, pc);
       view(pc, pv_seg, pv);
-      p_live = starts_before_end(pc, pv);
-      if (p_live) {
-        p_st = unit_stages(pc, pv);
-        pt = pc.k / pv.groups;
-        pg = pc.k - pt * pv.groups;
-      } else {
-        p_st = 0;
-      }
+      p_st = unit_stages(pc, pv);
+      pt = pc.k / pv.groups;
+      pg = pc.k - pt * pv.groups;
+      p_tma = unit_tma(pv, pg);
     }
   };
-  while (p_live && n_issued < kBLStages) issue_next();
+  while (n_issued < total && n_issued < kBLStages) issue_next();
 
   int64_t n_done = 0;
   bool aborted = false;
@@ -1058,21 +1082,21 @@ __global__ void __launch_bounds__(kBLWarps * 32) batched_lanes_kernel(const Batc
   int cv_seg = -1;
   LaneSeg cv;
   view(cu, cv_seg, cv);
-  while (starts_before_end(cu, cv) && !aborted) {
+  int j0 = first_j;
+  while (n_done < total && !aborted) {
     const LaneSeg& S = cv;
     const int64_t groups = S.groups;
     const int64_t t = cu.k / groups, g = cu.k - t * groups;
-    const int st_n = unit_stages(cu, cv);
+    const int st_n = (int)min((int64_t)unit_stages(cu, cv), j0 + total - n_done);  // the unit's, or up to the run's end
     const int64_t f = g * 32 + lane;
     const bool live = f < S.n_frames;
-    // quad rows: this lane's float offset into its box row; lanes past the
-    // last whole quad row read from global memory
+    const int tma = unit_tma(cv, g);
+    // quad rows: this lane's float offset into its box row
     const int quad_off = (int)(((int64_t)(lane & 3) * 3 * S.n_atoms) & 3);
-    const bool quad_tail = S.tma == 2 && f >= (S.n_frames & ~int64_t(3));
     double acc[15];
 #pragma unroll
     for (int e = 0; e < 15; ++e) acc[e] = 0.0;
-    for (int j = 0; j < st_n; ++j) {
+    for (int j = j0; j < st_n; ++j) {
       const int slot = (int)(n_done % kBLStages);
       const uint32_t parity = (uint32_t)((n_done / kBLStages) & 1);
       if (!mbar_wait(&full[slot], parity, B.status, kStatusTimeoutFull, abort_flag)) {
@@ -1083,54 +1107,59 @@ __global__ void __launch_bounds__(kBLWarps * 32) batched_lanes_kernel(const Batc
       const int nv = (int)min((int64_t)32, S.n_atoms - a0);
       const unsigned char* st = ring + slot * kBLXStage;
       const double* ys = reinterpret_cast<const double*>(yring + slot * kBLYBytes);
-      auto add = [&](double x0, double x1, double x2, int a) {
-        const double y0 = ys[3 * a], y1 = ys[3 * a + 1], y2 = ys[3 * a + 2];
+      auto add = [&](double x0, double x1, double x2, double y0, double y1, double y2) {
         acc[0] += x0; acc[1] += x1; acc[2] += x2;
         acc[3] = fma(x0, x0, acc[3]); acc[4] = fma(x1, x1, acc[4]); acc[5] = fma(x2, x2, acc[5]);
         acc[6] = fma(x0, y0, acc[6]);  acc[7] = fma(x0, y1, acc[7]);  acc[8] = fma(x0, y2, acc[8]);
         acc[9] = fma(x1, y0, acc[9]);  acc[10] = fma(x1, y1, acc[10]); acc[11] = fma(x1, y2, acc[11]);
         acc[12] = fma(x2, y0, acc[12]); acc[13] = fma(x2, y1, acc[13]); acc[14] = fma(x2, y2, acc[14]);
       };
-      if (live && S.tma == 1) {
-        // 4 atoms = 3 swizzled 16-byte chunks of this lane's 128-byte row in each box
+      if (live && tma == 1) {
+        // 4 atoms = 3 swizzled 16-byte chunks of this lane's 128-byte row in each box;
+        // atoms past the frame's end arrive as zeros and add nothing
         const unsigned char* row = st + lane * 128;
         const int sw = lane & 7;
         auto chunk = [&](int c) -> float4 {
           return *reinterpret_cast<const float4*>(row + (c >> 3) * 4096 + (((c & 7) ^ sw) << 4));
         };
+        const double2* yb = reinterpret_cast<const double2*>(ys);
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
           if (4 * m >= nv) break;
           const float4 p = chunk(3 * m), q = chunk(3 * m + 1), r = chunk(3 * m + 2);
-          add(p.x, p.y, p.z, 4 * m);
-          if (4 * m + 1 < nv) add(p.w, q.x, q.y, 4 * m + 1);
-          if (4 * m + 2 < nv) add(q.z, q.w, r.x, 4 * m + 2);
-          if (4 * m + 3 < nv) add(r.y, r.z, r.w, 4 * m + 3);
+          const double2 y01 = yb[6 * m + 0], y23 = yb[6 * m + 1], y45 = yb[6 * m + 2];
+          const double2 y67 = yb[6 * m + 3], y89 = yb[6 * m + 4], yab = yb[6 * m + 5];
+          add(p.x, p.y, p.z, y01.x, y01.y, y23.x);
+          add(p.w, q.x, q.y, y23.y, y45.x, y45.y);
+          add(q.z, q.w, r.x, y67.x, y67.y, y89.x);
+          add(r.y, r.z, r.w, y89.y, yab.x, yab.y);
         }
       } else if (live) {
         const float* xr;
-        if (S.tma == 2 && !quad_tail) {
+        if (tma == 2) {
           xr = reinterpret_cast<const float*>(st + (lane & 3) * kBLQuadBox + (lane >> 2) * kBLRow) + quad_off;
-        } else if (S.tma == 2) {
-          xr = S.coords + ((size_t)f * S.n_atoms + a0) * 3;
         } else {
           const int head = (int)(((uint64_t)(f * S.n_atoms + a0) * 12ull) & 15ull);
           xr = reinterpret_cast<const float*>(st + lane * kBLRow + head);
         }
 #pragma unroll 4
-        for (int a = 0; a < nv; ++a) add(xr[3 * a], xr[3 * a + 1], xr[3 * a + 2], a);
+        for (int a = 0; a < nv; ++a) add(xr[3 * a], xr[3 * a + 1], xr[3 * a + 2], ys[3 * a], ys[3 * a + 1], ys[3 * a + 2]);
       }
       ++n_done;
       __syncwarp();
-      if (p_live) issue_next();
+      if (n_issued < total) issue_next();
     }
     if (aborted) break;
     if (live) {
-      double2* rec = reinterpret_cast<double2*>(B.partial + (size_t)(S.item0 + t * S.n_frames + f) * kStatDoubles);
+      double2* rec = reinterpret_cast<double2*>(
+          j0 == 0 ? B.partial + (size_t)(S.item0 + t * S.n_frames + f) * kStatDoubles
+                  : B.lane_extra + (size_t)(gw * 32 + lane) * kStatDoubles);
 #pragma unroll
       for (int e = 0; e < 7; ++e) rec[e] = make_double2(acc[2 * e], acc[2 * e + 1]);
       rec[7] = make_double2(acc[14], 0.0);
     }
+    j0 = 0;
+    if (n_done == total) break;
     ++cu.k;
     lane_skip_empty(B, cu);
     view(cu, cv_seg, cv);
@@ -1151,6 +1180,31 @@ __global__ void __launch_bounds__(kBLWarps * 32) batched_lanes_kernel(const Batc
   }
 }
 
+// Adds the extra records of the units that several warps share to the units' records,
+// in warp order: the warp whose extra is a unit's first adds them all.
+__global__ void __launch_bounds__(256) batched_lanes_fold(const BatchLaunch B) {
+  const int64_t nw = B.lane_warps, w = (int64_t)blockIdx.x + 1;
+  const int64_t c = B.total_lane_stages * w / nw;
+  int j = 0;
+  const LaneCur u = lane_unit_of(B, c, j);
+  const int64_t unit0 = c - j;  // the unit's first stage
+  if (j == 0 || B.total_lane_stages * (w - 1) / nw > unit0) return;
+  const BatchSeg& S = B.segs[u.seg];
+  const int64_t end = unit0 + (u.k < S.lane_full_units ? S.lane_unit_stages : S.lane_last_stages);
+  const int64_t groups = (S.n_frames + 31) / 32, t = u.k / groups, f0 = (u.k - t * groups) * 32;
+  // 512 doubles: 32 frames x 16 sums, a double2 per thread
+  const int i = threadIdx.x, row = i >> 3;
+  if (f0 + row >= S.n_frames) return;
+  double2* rec = reinterpret_cast<double2*>(B.partial + (size_t)(S.item0 + t * S.n_frames + f0) * kStatDoubles) + i;
+  double2 v = *rec;
+  for (int64_t x = w; x < nw && B.total_lane_stages * x / nw < end; ++x) {
+    const double2 e = reinterpret_cast<const double2*>(B.lane_extra + (size_t)x * (32 * kStatDoubles))[i];
+    v.x += e.x;
+    v.y += e.y;
+  }
+  *rec = v;
+}
+
 template <int APT>
 cudaError_t launch_lanes(const BatchLaunch& B, int grid, cudaStream_t s) {
   auto kern = batched_lanes_kernel<APT>;
@@ -1163,7 +1217,12 @@ cudaError_t launch_lanes(const BatchLaunch& B, int grid, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
-  kern<<<grid, kBLWarps * 32, kBLSmemBytes, s>>>(B);
+  BatchLaunch K = B;
+  K.lane_warps = std::min<int64_t>((int64_t)grid * kBLWarps, B.total_lane_stages);
+  kern<<<grid, kBLWarps * 32, kBLSmemBytes, s>>>(K);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  if (K.lane_warps > 1) batched_lanes_fold<<<(unsigned)(K.lane_warps - 1), 256, 0, s>>>(K);
   return cudaGetLastError();
 }
 
@@ -1271,7 +1330,7 @@ int batched_tile_atoms(int apt) { return kConsumerThreads * apt; }
 cudaError_t batched_enqueue(const BatchPlan& P, bool with_grad, cudaStream_t s) {
   BatchLaunch B = P.launch;
   cudaError_t e;
-  batched_ref_prep<<<P.n_segs, 256, 0, s>>>(P.segs_dev);
+  batched_ref_prep<<<P.n_segs, kPrepThreads, 0, s>>>(P.segs_dev);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (P.variant == kBatchFrames) {
     if (B.total_groups == 0) return cudaSuccess;
@@ -1288,7 +1347,7 @@ cudaError_t batched_enqueue(const BatchPlan& P, bool with_grad, cudaStream_t s) 
     if (e != cudaSuccess) return e;
   }
   if (B.total_frames > 0) {
-    batched_finalize<<<(unsigned)((B.total_frames + 255) / 256), 256, 0, s>>>(B);
+    batched_finalize<<<(unsigned)((B.total_frames + kFinWarps * 32 - 1) / (kFinWarps * 32)), kFinWarps * 32, 0, s>>>(B);
     batched_refine<<<(unsigned)std::min<int64_t>(B.total_frames, 148), 256, 0, s>>>(B);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -1305,7 +1364,7 @@ int batched_grid(int apt, bool backward, int sm_count, int64_t items) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)sm_count * occ));
 }
 
-int batched_lanes_grid(int sm_count, int64_t units) {
+int batched_lanes_grid(int sm_count, int64_t stages) {
   static int occ = 0;
   if (occ == 0) {
     cudaFuncSetAttribute(batched_lanes_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBLSmemBytes);
@@ -1315,8 +1374,12 @@ int batched_lanes_grid(int sm_count, int64_t units) {
       b = 1;
     occ = std::max(b, 1);
   }
-  const int64_t by_units = (units + kBLWarps - 1) / kBLWarps;
-  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count * occ, by_units));
+  const int64_t by_stages = stages / kBLWarps + 1;
+  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count * occ, by_stages));
+}
+
+size_t batched_lanes_extra_bytes(int sm_count) {
+  return (size_t)batched_lanes_grid(sm_count, INT64_MAX) * kBLWarps * 32 * kStatDoubles * sizeof(double);
 }
 
 int batched_frame_grid(int apt, bool with_grad, int sm_count, int64_t groups) {

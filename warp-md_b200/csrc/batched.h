@@ -25,11 +25,11 @@ struct BatchSeg {
   int64_t n_groups;     //   groups of this trajectory (m_group frames each, the last may be short)
   int64_t cost0;        //   estimated cost of all groups before this trajectory's
   int64_t group_cost;   //   estimated cost of one full group
-  int64_t lane_unit_cost;  // lanes layout: estimated cost of a (tile, 32-frame group) unit of a whole tile
-  int64_t lane_last_cost;  //   ... and of a unit of the last tile (the only one when n_atoms <= tile)
+  int64_t lane_unit_stages;  // lanes layout: 32-atom stages of a (tile, 32-frame group) unit of a whole tile
+  int64_t lane_last_stages;  //   ... and of a unit of the last tile (the only one when n_atoms <= tile)
   int64_t lane_full_units; //   units of the whole tiles, (n_tiles - 1) x ceil(n_frames / 32); tile-major
   int64_t lane_units;      //   units of this trajectory (n_tiles x ceil(n_frames / 32))
-  int64_t lane_cost0;      //   estimated cost of all units before this trajectory's
+  int64_t lane_stage0;     //   stages of all trajectories before this one
   int n_tiles;
   int m_group;          //   frames per group
   int tma;              // lanes layout forward: 0 per-lane bulk copies, 1 frame rows, 2 quad rows (tensor map)
@@ -46,7 +46,9 @@ struct BatchLaunch {
   int64_t total_frames = 0;
   int64_t total_groups = 0;          // frame-major layout
   int64_t total_cost = 0;
-  int64_t total_lane_cost = 0;       // lanes layout
+  int64_t total_lane_stages = 0;     // lanes layout
+  int64_t lane_warps = 0;            //   active warps (set at launch)
+  double* lane_extra = nullptr;      //   [warps][32][16], batched_lanes_extra_bytes
   double* partial = nullptr;         // [total_items][16]
   double* rot = nullptr;             // [total_frames][16] (with gradients): R, xbar, 1/(n rmsd)
   double* refine = nullptr;          // [total_frames][16]
@@ -97,7 +99,8 @@ bool batched_encode_maps(std::vector<BatchSeg>& segs, CUtensorMap* maps, std::st
 int batched_tile_atoms(int apt);
 int batched_grid(int apt, bool backward, int sm_count, int64_t items);
 int batched_frame_grid(int apt, bool with_grad, int sm_count, int64_t groups);
-int batched_lanes_grid(int sm_count, int64_t units);
+int batched_lanes_grid(int sm_count, int64_t stages);
+size_t batched_lanes_extra_bytes(int sm_count);
 // Enqueues the whole batched pipeline on s (no allocation, no host sync).
 cudaError_t batched_enqueue(const BatchPlan& P, bool with_grad, cudaStream_t s);
 

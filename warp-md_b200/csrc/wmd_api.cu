@@ -1841,10 +1841,10 @@ static int64_t batch_yc_doubles(int64_t n_atoms) { return (n_atoms * 3 + 1) / 2 
 
 static int64_t build_segs(const std::vector<wmd_batch_desc>& d, int apt, double* yc_base, bool with_grad,
                           std::vector<wmd::BatchSeg>& segs, int64_t* total_frames, int64_t* total_groups,
-                          int64_t* total_cost, int64_t* total_lane_cost) {
+                          int64_t* total_cost, int64_t* total_lane_stages) {
   const int tile = wmd::batched_tile_atoms(apt);
   segs.assign(d.size(), wmd::BatchSeg{});
-  int64_t items = 0, frames = 0, yoff = 0, groups = 0, cost = 0, lane_cost = 0;
+  int64_t items = 0, frames = 0, yoff = 0, groups = 0, cost = 0, lane_stages = 0;
   for (size_t i = 0; i < d.size(); ++i) {
     wmd::BatchSeg& g = segs[i];
     g.coords = d[i].coords;
@@ -1856,23 +1856,20 @@ static int64_t build_segs(const std::vector<wmd_batch_desc>& d, int apt, double*
     g.n_tiles = (int)((d[i].n_atoms + tile - 1) / tile);
     g.yc = yc_base + yoff;
     yoff += batch_yc_doubles(d[i].n_atoms);
-    // lanes layout: (tile, 32-frame group) units, tile-major; cost ~ the
-    // tile's atom-frames plus a per-stage overhead of about 8 atoms' work and a
-    // per-unit one of about a stage (the partial records); the last tile holds
-    // the remainder of the atoms
-    g.lane_cost0 = lane_cost;
-    auto unit_cost = [](int64_t at) { return 32 * (at + 8 * ((at + 31) / 32) + 32); };
+    // lanes layout: (tile, 32-frame group) units of 32-atom stages, tile-major; the
+    // last tile holds the remainder of the atoms
+    g.lane_stage0 = lane_stages;
     if (g.n_atoms > 0 && g.n_frames > 0) {
       const int64_t groups_f = (g.n_frames + 31) / 32;
       g.lane_units = (int64_t)g.n_tiles * groups_f;
       g.lane_full_units = (int64_t)(g.n_tiles - 1) * groups_f;
-      g.lane_unit_cost = unit_cost(tile);
-      g.lane_last_cost = unit_cost(g.n_atoms - (int64_t)(g.n_tiles - 1) * tile);
+      g.lane_unit_stages = tile / 32;
+      g.lane_last_stages = (g.n_atoms - (int64_t)(g.n_tiles - 1) * tile + 31) / 32;
     } else {
       g.lane_units = g.lane_full_units = 0;
-      g.lane_unit_cost = g.lane_last_cost = 1;
+      g.lane_unit_stages = g.lane_last_stages = 1;
     }
-    lane_cost += g.lane_full_units * g.lane_unit_cost + (g.lane_units - g.lane_full_units) * g.lane_last_cost;
+    lane_stages += g.lane_full_units * g.lane_unit_stages + (g.lane_units - g.lane_full_units) * g.lane_last_stages;
     g.item0 = items;
     g.frame0 = frames;
     items += (int64_t)g.n_tiles * g.n_frames;
@@ -1899,7 +1896,7 @@ static int64_t build_segs(const std::vector<wmd_batch_desc>& d, int apt, double*
   *total_frames = frames;
   *total_groups = groups;
   *total_cost = cost;
-  *total_lane_cost = lane_cost;
+  *total_lane_stages = lane_stages;
   return items;
 }
 
@@ -1939,9 +1936,9 @@ WMD_EXPORT int wmd_batched_prepare(wmd_ctx* ctx, const wmd_batch_desc* descs, in
   double* yc = static_cast<double*>(ctx->b_yc.ptr);
   // the padding after every block must read as zeros
   CU(cudaMemset(yc, 0, (size_t)std::max<int64_t>(sum_atoms, 2) * sizeof(double)), "memset");
-  int64_t groups4 = 0, groups8 = 0, cost4 = 0, cost8 = 0, lcost4 = 0, lcost8 = 0;
-  const int64_t items4 = build_segs(d, 4, yc, with_grad != 0, s4, &frames4, &groups4, &cost4, &lcost4);
-  const int64_t items8 = build_segs(d, 8, yc, with_grad != 0, s8, &frames8, &groups8, &cost8, &lcost8);
+  int64_t groups4 = 0, groups8 = 0, cost4 = 0, cost8 = 0, lst4 = 0, lst8 = 0;
+  const int64_t items4 = build_segs(d, 4, yc, with_grad != 0, s4, &frames4, &groups4, &cost4, &lst4);
+  const int64_t items8 = build_segs(d, 8, yc, with_grad != 0, s8, &frames8, &groups8, &cost8, &lst8);
   const int64_t frames = frames4;
   const size_t rec = wmd::kStatDoubles * sizeof(double);
   // the lanes layout's tensor maps (one per trajectory; the same for both tile shapes)
@@ -1955,7 +1952,8 @@ WMD_EXPORT int wmd_batched_prepare(wmd_ctx* ctx, const wmd_batch_desc* descs, in
        "upload tensor maps");
   }
   if ((rc = ensure(ctx, ctx->b_segs, std::max<size_t>(1, (size_t)n_traj) * sizeof(wmd::BatchSeg))) ||
-      (rc = ensure(ctx, ctx->b_partial, (size_t)std::max<int64_t>(1, std::max(items4, items8)) * rec)) ||
+      (rc = ensure(ctx, ctx->b_partial, (size_t)std::max<int64_t>(1, std::max(items4, items8)) * rec +
+                                            wmd::batched_lanes_extra_bytes(ctx->sm_count))) ||
       (rc = ensure(ctx, ctx->b_refine, (size_t)std::max<int64_t>(1, frames) * rec)) ||
       (rc = ensure(ctx, ctx->b_count, sizeof(unsigned), true)))
     return rc;
@@ -1968,6 +1966,7 @@ WMD_EXPORT int wmd_batched_prepare(wmd_ctx* ctx, const wmd_batch_desc* descs, in
   P.launch.n_segs = n_traj;
   P.launch.total_frames = frames;
   P.launch.partial = static_cast<double*>(ctx->b_partial.ptr);
+  P.launch.lane_extra = P.launch.partial + std::max<int64_t>(1, std::max(items4, items8)) * wmd::kStatDoubles;
   P.launch.rot = with_grad ? static_cast<double*>(ctx->b_rot.ptr) : nullptr;
   P.launch.refine = static_cast<double*>(ctx->b_refine.ptr);
   P.launch.refine_count = static_cast<unsigned*>(ctx->b_count.ptr);
@@ -1985,11 +1984,9 @@ WMD_EXPORT int wmd_batched_prepare(wmd_ctx* ctx, const wmd_batch_desc* descs, in
     P.launch.total_items = apt == 4 ? items4 : items8;
     P.launch.total_groups = apt == 4 ? groups4 : groups8;
     P.launch.total_cost = apt == 4 ? cost4 : cost8;
-    P.launch.total_lane_cost = apt == 4 ? lcost4 : lcost8;
+    P.launch.total_lane_stages = apt == 4 ? lst4 : lst8;
     if (variant == wmd::kBatchLanes) {
-      int64_t units = 0;
-      for (const wmd::BatchSeg& g : sv) units += g.lane_units;
-      P.grid_fwd = wmd::batched_lanes_grid(ctx->sm_count, units);
+      P.grid_fwd = wmd::batched_lanes_grid(ctx->sm_count, P.launch.total_lane_stages);
       P.grid_bwd = wmd::batched_grid(apt, true, ctx->sm_count, P.launch.total_items);
     } else if (variant == wmd::kBatchFrames) {
       P.grid_fwd = wmd::batched_frame_grid(apt, with_grad != 0, ctx->sm_count, P.launch.total_groups);
