@@ -26,8 +26,9 @@ cudaError_t kmeans_features(const float* coords, int64_t n_frames, int64_t n_ato
 cudaError_t kmeans_gather(const double* feat, int64_t nf, const int64_t* idx, int k, double* centers, cudaStream_t s);
 cudaError_t kmeans_assign(const double* feat, int64_t n, int64_t nf, const double* centers, int k, int* labels,
                           double* dist_own, cudaStream_t s);
-cudaError_t kmeans_sums(const double* feat, int64_t n, int64_t nf, const int* labels, int k, double* sums, int* counts,
-                        cudaStream_t s);
+// members [n]: the samples cluster after cluster, in index order (starts [k], counts [k])
+cudaError_t kmeans_sums(const double* feat, int64_t n, int64_t nf, const int* labels, int k, int* members, int64_t* starts,
+                        double* sums, int* counts, cudaStream_t s);
 cudaError_t kmeans_centers(const double* feat, int64_t nf, const double* sums, const int* counts, const int64_t* reseed,
                            int k, const double* old_c, double* new_c, double* shift, cudaStream_t s);
 // Final sizes (from labels) and per-cluster nearest member to the final center

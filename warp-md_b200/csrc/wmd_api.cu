@@ -1768,12 +1768,12 @@ WMD_EXPORT int wmd_cluster_kmeans(wmd_ctx* ctx, const float* coords, int64_t n_f
     return WMD_OK;
   });
   if (rc) return rc;
-  // work: centers x2, sums [K][nf]; labels [N]; counts [K]; reseed [K]; shift [K];
+  // work: centers x2, sums [K][nf]; labels [N]; counts [K]; members [N], starts [K]; reseed [K]; shift [K];
   // dist [N]; best [K]; sizes, centroids [K]
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
   const size_t cbytes = al((size_t)K * nf * 8);
-  const size_t total = 3 * cbytes + al(N * 4) + al(K * 4) + al(K * 8) + al(K * 8) + al(N * 8) + al(K * 8) +
-                       2 * al(K * 4);
+  const size_t total = 3 * cbytes + al(N * 4) + al(K * 4) + al(N * 4) + al(K * 8) + al(K * 8) + al(K * 8) + al(N * 8) +
+                       al(K * 8) + 2 * al(K * 4);
   if ((rc = ensure(ctx, ctx->km_work, total))) return rc;
   char* w = static_cast<char*>(ctx->km_work.ptr);
   double* cen_a = reinterpret_cast<double*>(w);
@@ -1783,6 +1783,8 @@ WMD_EXPORT int wmd_cluster_kmeans(wmd_ctx* ctx, const float* coords, int64_t n_f
   auto take = [&](size_t b) { char* p = w + off; off += al(b); return p; };
   int* dlabels = reinterpret_cast<int*>(take(N * 4));
   int* dcounts = reinterpret_cast<int*>(take(K * 4));
+  int* dmembers = reinterpret_cast<int*>(take(N * 4));
+  int64_t* dstarts = reinterpret_cast<int64_t*>(take(K * 8));
   int64_t* dreseed = reinterpret_cast<int64_t*>(take(K * 8));
   double* dshift = reinterpret_cast<double*>(take(K * 8));
   double* ddist = reinterpret_cast<double*>(take(N * 8));
@@ -1805,7 +1807,7 @@ WMD_EXPORT int wmd_cluster_kmeans(wmd_ctx* ctx, const float* coords, int64_t n_f
   std::vector<double> shift((size_t)K);
   for (int64_t it = 0; it < iters; ++it) {
     CU(wmd::kmeans_assign(feat, N, nf, cen_a, (int)K, dlabels, nullptr, s), "kmeans assign");
-    CU(wmd::kmeans_sums(feat, N, nf, dlabels, (int)K, sums, dcounts, s), "kmeans sums");
+    CU(wmd::kmeans_sums(feat, N, nf, dlabels, (int)K, dmembers, dstarts, sums, dcounts, s), "kmeans sums");
     CU(cudaMemcpyAsync(counts.data(), dcounts, (size_t)K * 4, cudaMemcpyDeviceToHost, s), "D2H");
     CU(cudaStreamSynchronize(s), "synchronize");
     for (int64_t c = 0; c < K; ++c)
