@@ -311,8 +311,9 @@ int pairwise_run(PairwiseWorkspace& w, int sm_count, const float* coords, int64_
   const bool tc64 = f64 && n_sel <= kTc64MaxAtoms && simt_waves * n_sel >= 160;
   const bool zeros = n_sel < 2 || n_frames < 2;  // all zeros (plan.rs:604-610)
   cudaError_t e;
-  // the 40-bit form of a whole matrix writes every entry itself
-  if (zeros || !tc64 || w.parts > 1) {
+  // the tensor-core forms of a whole matrix write every entry themselves
+  const bool tc = tc64 || mode == WMD_MODE_I8X3 || mode == WMD_MODE_I8X2;
+  if (zeros || !tc || w.parts > 1) {
     if ((e = cudaMemsetAsync(out, 0, (size_t)n_frames * n_frames * sizeof(float), s)) != cudaSuccess)
       return cuda_fail(e, "");
   }
