@@ -4,9 +4,10 @@
 // copies the centred coordinates back: three synchronous copies and an
 // allocation, ~85 us for 2,000 atoms against 53 us for the value-and-gradient
 // kernel that follows.  Here one CTA does the same on the caller's stream,
-// latency-bound (two passes, two block reductions): 8 us for 2,000 atoms, and
+// latency-bound (two passes, two block reductions): 6.5 us for 2,000 atoms (8.3 with
+// the loads of one atom in flight), and
 // nothing waits for it on the host (rmsd_value_and_grad of 4,096 x 2,000 with a
-// new reference 141 -> 66 us).  More CTAs would need a grid barrier between the
+// new reference 141 -> 63 us).  More CTAs would need a grid barrier between the
 // passes.
 //
 // Every sum carries the rounding error of its additions along (Knuth's TwoSum), as
@@ -42,6 +43,24 @@ __device__ __forceinline__ void tree_add(ExactSum& v, int o) {
   v.merge(s2, c2);
 }
 
+// fn(k, y) for this thread's atoms in order, kRefAhead of them loaded at a time.
+constexpr int kRefAhead = 4;
+
+template <int STRIDE, class Fn>
+__device__ __forceinline__ void each_atom(const float* __restrict__ ref, int64_t n, Fn fn) {
+  for (int64_t k0 = threadIdx.x; k0 < n; k0 += kRefAhead * kRefThreads) {
+    float y[kRefAhead][3];
+#pragma unroll
+    for (int u = 0; u < kRefAhead; ++u)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        y[u][c] = k0 + u * kRefThreads < n ? __ldg(ref + (k0 + u * kRefThreads) * STRIDE + c) : 0.f;
+#pragma unroll
+    for (int u = 0; u < kRefAhead; ++u)
+      if (k0 + u * kRefThreads < n) fn(k0 + u * kRefThreads, y[u]);
+  }
+}
+
 template <int STRIDE>
 __global__ void __launch_bounds__(kRefThreads) ref_prep_kernel(const float* __restrict__ ref, int64_t n,
                                                                double* __restrict__ yc, double* __restrict__ scal) {
@@ -49,9 +68,10 @@ __global__ void __launch_bounds__(kRefThreads) ref_prep_kernel(const float* __re
   __shared__ double red[kWarps][4][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   ExactSum m[3];
-  for (int64_t k = threadIdx.x; k < n; k += kRefThreads)
+  each_atom<STRIDE>(ref, n, [&](int64_t, const float (&y)[3]) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) m[c].add((double)ref[k * STRIDE + c]);
+    for (int c = 0; c < 3; ++c) m[c].add((double)y[c]);
+  });
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
 #pragma unroll
@@ -73,14 +93,15 @@ __global__ void __launch_bounds__(kRefThreads) ref_prep_kernel(const float* __re
   }
   __syncthreads();  // red is written again
   ExactSum e[4];  // sum of y_c, sum |y_c|^2
-  for (int64_t k = threadIdx.x; k < n; k += kRefThreads)
+  each_atom<STRIDE>(ref, n, [&](int64_t k, const float (&y)[3]) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const double d = (double)ref[k * STRIDE + c] - mean[c];
+      const double d = (double)y[c] - mean[c];
       yc[k * 3 + c] = d;
       e[c].add(d);
       e[3].add(d * d);
     }
+  });
   // 32 zero atoms after the reference: the frames-across-lanes kernels copy
   // whole 32-atom blocks of it
   for (int64_t k = n * 3 + threadIdx.x; k < (n + 32) * 3; k += kRefThreads) yc[k] = 0.0;
