@@ -81,6 +81,8 @@ __device__ __forceinline__ void item_epilogue(const FrameLaunch& L, const double
 // 4,000 frames x 196 tiles, with 16 in flight 14.5 us.
 template <int MODE>
 __global__ void __launch_bounds__(256) rmsd_finalize_kernel(const FrameLaunch L, int n_tiles) {
+  depend_wait();
+  depend_launch();
   const int64_t f = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (f >= L.n_frames) return;
   const int lane = threadIdx.x & 31;
@@ -149,6 +151,7 @@ __global__ void __launch_bounds__(kThreads, 3) rmsd_frames_kernel(const FrameLau
   double* red = reinterpret_cast<double*>(smem + G::kRedOffset);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + G::kAbortOffset);
 
+  if (MODE != kBwd) depend_launch();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t n_sel = L.ref.n_sel;
   const int64_t F = L.n_frames;
@@ -379,6 +382,7 @@ __global__ void rmsd_bwd_prologue(const double* __restrict__ stats, const float*
 template <int STRIDE>
 __global__ void __launch_bounds__(256) rmsd_refine_kernel(const FrameLaunch L) {
   __shared__ double red[8];
+  depend_wait();
   const unsigned count = *L.refine_count;
   for (unsigned rix = blockIdx.x; rix < count; rix += gridDim.x) {
     residual_rmsd<STRIDE>(L, L.refine + (size_t)rix * kStatDoubles, red);
@@ -406,6 +410,7 @@ constexpr int gather_ctas(int mode) { return mode == kFwdW ? 4 : 6; }
 
 template <int STRIDE, int MODE>
 __global__ void __launch_bounds__(kGatherThreads, gather_ctas(MODE)) rmsd_gather_kernel(const FrameLaunch L, int tile) {
+  depend_launch();
   const int lane = threadIdx.x & 31;
   const int64_t gw = ((int64_t)blockIdx.x * kGatherThreads + threadIdx.x) >> 5;
   const int64_t n_warps = (int64_t)gridDim.x * (kGatherThreads / 32);
@@ -580,15 +585,13 @@ cudaError_t launch_rmsd_forward(const FrameLaunch& L, cudaStream_t s) {
   } else {
     if ((e = L.align ? dispatch<kFwdFit>(K, s) : dispatch<kFwdRaw>(K, s)) != cudaSuccess) return e;
     const unsigned blocks = (unsigned)((L.n_frames + 7) / 8);
-    if (L.align) rmsd_finalize_kernel<kFwdFit><<<blocks, 256, 0, s>>>(K, frame_tiles(L));
-    else rmsd_finalize_kernel<kFwdRaw><<<blocks, 256, 0, s>>>(K, frame_tiles(L));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_dependent(L.align ? rmsd_finalize_kernel<kFwdFit> : rmsd_finalize_kernel<kFwdRaw>, blocks, 256, 0, s, K,
+                         frame_tiles(L));
+    if (e != cudaSuccess) return e;
   }
   if (!refine) return cudaSuccess;
   const int blocks = (int)std::min<int64_t>(L.n_frames, 148);
-  if (L.stride == 4) rmsd_refine_kernel<4><<<blocks, 256, 0, s>>>(K);
-  else rmsd_refine_kernel<3><<<blocks, 256, 0, s>>>(K);
-  return cudaGetLastError();
+  return launch_dependent(L.stride == 4 ? rmsd_refine_kernel<4> : rmsd_refine_kernel<3>, blocks, 256, 0, s, K);
 }
 
 cudaError_t launch_rmsd_stream(const FrameLaunch& L, cudaStream_t s) {

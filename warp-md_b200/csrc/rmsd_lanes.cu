@@ -276,6 +276,7 @@ template <int STRIDE, bool RAW, bool W, bool QUAD = false>
 __global__ void __launch_bounds__(kLaneWarps * 32) rmsd_lanes_kernel(const __grid_constant__ CUtensorMap map,
                                                                      const FrameLaunch L) {
   using G = typename PickGeo<QUAD, STRIDE>::type;
+  depend_launch();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -454,6 +455,8 @@ constexpr int kFinalizeWarps = 16;
 template <int MODE>
 __global__ void __launch_bounds__(kFinalizeWarps * 32) lanes_finalize_kernel(const FrameLaunch L) {
   extern __shared__ double red[];  // [kFinalizeWarps][15][32]
+  depend_wait();
+  depend_launch();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const LaneSplit split(L);
   const int64_t g = blockIdx.x;
@@ -556,8 +559,7 @@ cudaError_t launch_lanes(const FrameLaunch& L, cudaStream_t s) {
     if ((e = cudaFuncSetAttribute(fin, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinBytes)) != cudaSuccess) return e;
     fin_done[dev] = true;
   }
-  fin<<<(unsigned)((L.n_frames + 31) / 32), kFinalizeWarps * 32, kFinBytes, s>>>(L);
-  return cudaGetLastError();
+  return launch_dependent(fin, (unsigned)((L.n_frames + 31) / 32), kFinalizeWarps * 32, kFinBytes, s, L);
 }
 
 // Packed xyz frames whose stride is not a multiple of 16 bytes, streamed as

@@ -41,6 +41,7 @@ constexpr int kFinFrames = 8;
 __global__ void __launch_bounds__(32) superpose_finalize_kernel(const FrameLaunch L, int n_tiles, int norotate,
                                                                 double* __restrict__ xf64, float* __restrict__ xf32) {
   __shared__ double st[kFinFrames][17];
+  depend_wait();
   const int lane = threadIdx.x;
   const int64_t base = (int64_t)blockIdx.x * kFinFrames;
 #pragma unroll
@@ -247,8 +248,7 @@ __global__ void __launch_bounds__(kThreads, 4) superpose_apply_staged(const floa
 cudaError_t launch_superpose_finalize(const FrameLaunch& L, int norotate, double* xf64, float* xf32, cudaStream_t s) {
   if (L.n_frames == 0) return cudaSuccess;
   const unsigned blocks = (unsigned)((L.n_frames + kFinFrames - 1) / kFinFrames);
-  superpose_finalize_kernel<<<blocks, 32, 0, s>>>(L, frame_tiles(L), norotate, xf64, xf32);
-  return cudaGetLastError();
+  return launch_dependent(superpose_finalize_kernel, blocks, 32, 0, s, L, frame_tiles(L), norotate, xf64, xf32);
 }
 
 cudaError_t launch_superpose_apply(const float* coords, int64_t n_frames, int64_t n_atoms, int stride,
