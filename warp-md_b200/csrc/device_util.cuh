@@ -150,6 +150,10 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
 // 2,400 x 1,000 atoms 21.7 / 18.6, 1,000 x 10,000 40.0 / 35.0, 5,001 x 3,001 49.9 / 47.2,
 // 2,000 x 5,000 every tenth 35.6 / 30.7.
 __device__ __forceinline__ void depend_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Ties the read-only loads (ld.global.nc) through p to the wait before it: the
+// compiler may take what they read for constant over the kernel.
+template <class T>
+__device__ __forceinline__ void depend_read(T*& p) { asm volatile("" : "+l"(p)); }
 __device__ __forceinline__ void depend_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <class... P, class... A>

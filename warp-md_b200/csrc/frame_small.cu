@@ -26,10 +26,14 @@ constexpr int kSmallWarps = 8;
 constexpr int kSmallThreads = kSmallWarps * 32;
 
 template <int STRIDE, int MODE>
-__global__ void __launch_bounds__(kSmallThreads) rmsd_small_kernel(const FrameLaunch L) {
+__global__ void __launch_bounds__(kSmallThreads) rmsd_small_kernel(const FrameLaunch P) {
   __shared__ double red[kSmallWarps][16];
   __shared__ double rec[kStatDoubles];
   __shared__ unsigned queued;
+  FrameLaunch L = P;
+  depend_wait();  // for a reference centred just before (reference.cu)
+  depend_read(L.ref.yc);
+  depend_read(L.ref.scal);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t n = L.ref.n_sel;
   const double mean[3] = {MODE == kFwdRaw ? ref_mean(L.ref, 0) : 0.0, MODE == kFwdRaw ? ref_mean(L.ref, 1) : 0.0,
@@ -120,14 +124,11 @@ bool small_frames(const FrameLaunch& L) {
 
 cudaError_t launch_small_forward(const FrameLaunch& L, cudaStream_t s) {
   const unsigned grid = (unsigned)L.n_frames;
-  if (L.stride == 4) {
-    if (L.align) rmsd_small_kernel<4, kFwdFit><<<grid, kSmallThreads, 0, s>>>(L);
-    else rmsd_small_kernel<4, kFwdRaw><<<grid, kSmallThreads, 0, s>>>(L);
-  } else {
-    if (L.align) rmsd_small_kernel<3, kFwdFit><<<grid, kSmallThreads, 0, s>>>(L);
-    else rmsd_small_kernel<3, kFwdRaw><<<grid, kSmallThreads, 0, s>>>(L);
-  }
-  return cudaGetLastError();
+  if (L.stride == 4)
+    return launch_dependent(L.align ? rmsd_small_kernel<4, kFwdFit> : rmsd_small_kernel<4, kFwdRaw>, grid, kSmallThreads,
+                            0, s, L);
+  return launch_dependent(L.align ? rmsd_small_kernel<3, kFwdFit> : rmsd_small_kernel<3, kFwdRaw>, grid, kSmallThreads, 0,
+                          s, L);
 }
 
 cudaError_t launch_small_backward(const FrameLaunch& L, const double* stats, const float* grad_rmsd,

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kRefThreads) ref_prep_kernel(const float* __re
                                                                double* __restrict__ yc, double* __restrict__ scal) {
   constexpr int kWarps = kRefThreads / 32;
   __shared__ double red[kWarps][4][2];
+  depend_launch();  // the kernel that reads yc starts meanwhile
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   ExactSum m[3];
   each_atom<STRIDE>(ref, n, [&](int64_t, const float (&y)[3]) {

@@ -135,7 +135,8 @@ __device__ __forceinline__ float4* stage_chunk(unsigned char* st, int lane, int 
 template <int MODE>
 __global__ void __launch_bounds__(kVgThreads, 1) rmsd_vg_kernel(const __grid_constant__ CUtensorMap mx,
                                                                 const __grid_constant__ CUtensorMap mg,
-                                                                const VgArgs A) {
+                                                                const VgArgs P) {
+  VgArgs A = P;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -159,6 +160,9 @@ __global__ void __launch_bounds__(kVgThreads, 1) rmsd_vg_kernel(const __grid_con
     *any_flag = 0;
     fence_barrier_init();
   }
+  depend_wait();  // for a reference centred just before (reference.cu)
+  depend_read(A.yc);
+  depend_read(A.ref.scal);
   __syncthreads();
 
   // Ring counters: loads issued (lane 0) and stages consumed (all lanes).
@@ -507,8 +511,7 @@ cudaError_t launch_mode(const CUtensorMap& mx, const CUtensorMap& mg, const VgAr
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
-  kern<<<grid, kVgThreads, kVgSmemBytes, s>>>(mx, mg, A);
-  return cudaGetLastError();
+  return launch_dependent(kern, grid, kVgThreads, kVgSmemBytes, s, mx, mg, A);
 }
 
 }  // namespace
