@@ -2025,7 +2025,12 @@ WMD_EXPORT int wmd_batched_prepare(wmd_ctx* ctx, const wmd_batch_desc* descs, in
         CU(cudaEventSynchronize(e1), "synchronize");
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
-        if (best_ms < 0.f || ms < best_ms) {
+        // one run each, which repeats to ~2 %: 512-atom tiles (twice the records) have to
+        // beat the same layout's 1,024-atom tiles by more than that (30 trajectories,
+        // 277 million atom-frames: 1.87 against 1.98 ms when the runs are repeated, yet
+        // picked now and then)
+        const float margin = best_layout == layout && best_apt == 8 && apt == 4 ? 0.97f : 1.f;
+        if (best_ms < 0.f || ms < best_ms * margin) {
           best_ms = ms;
           best_apt = apt;
           best_layout = layout;
