@@ -120,7 +120,7 @@ __device__ __forceinline__ void batched_issue(const BatchSeg& s, int t, int64_t 
   if (rot) bulk_copy_g2s(dst + BGeo<APT>::kRecOffset, rot + (s.frame0 + f) * kStatDoubles, kStatDoubles * 8, bar);
 }
 
-template <int APT, int MODE>
+template <int APT>
 __global__ void __launch_bounds__(kThreads, 4) batched_stream_kernel(const BatchLaunch B) {
   using G = BGeo<APT>;
   constexpr int T = G::kTile;
@@ -143,8 +143,7 @@ __global__ void __launch_bounds__(kThreads, 4) batched_stream_kernel(const Batch
 
   Cursor pc;  // producer cursor (thread 0)
   int64_t issued = 0;
-  // the gradient pass stages each frame's rotation record with its coordinates
-  const double* rec_src = MODE == kBBwd ? B.rot : nullptr;
+  const double* rec_src = nullptr;
   if (tid == 0) {
     cursor_init(B, w0, pc);
     for (; issued < S - 1 && issued < n_items; ++issued) {
@@ -159,9 +158,7 @@ __global__ void __launch_bounds__(kThreads, 4) batched_stream_kernel(const Batch
   int s = 0;
   uint32_t phase = 0;
   for (int64_t i = 0; i < n_items; ++i) {
-    // forward: refill at the top of the iteration; backward: after the
-    // stage's gradient store has been issued (see below)
-    if (MODE == kBFwd && tid == 0 && issued < n_items) {
+    if (tid == 0 && issued < n_items) {
       const int sp = (int)(issued % S);
       batched_issue<APT>(B.segs[pc.seg], pc.t, pc.f, smem + sp * G::kStageBytes, &full[sp], rec_src);
       ++issued;
@@ -188,98 +185,38 @@ __global__ void __launch_bounds__(kThreads, 4) batched_stream_kernel(const Batch
     const float* xs = reinterpret_cast<const float*>(smem + s * G::kStageBytes) +
                       (int)(((uint64_t)(c.f * sg.n_atoms + a0) * 3) & 3ull);
     const int64_t gitem = w0 + i;
-    if (MODE == kBBwd) {
-      // dRMSD/dx is written over x in the stage (each thread its own atoms),
-      // then leaves by one bulk store of the tile's 16-byte-aligned middle and
-      // at most 2 x 3 scalar floats at its ends.
-      float* gs = const_cast<float*>(xs);
-      const bool has_grad = sg.grad != nullptr;
-      if (ok && has_grad) {
-        const double* rt = reinterpret_cast<const double*>(smem + s * G::kStageBytes + G::kRecOffset);
-        double R[9], cc[3];
+    double acc[16];
 #pragma unroll
-        for (int e = 0; e < 9; ++e) R[e] = rt[e];
-        cc[0] = rt[9]; cc[1] = rt[10]; cc[2] = rt[11];
-        const double scale = rt[12];
+    for (int e = 0; e < 16; ++e) acc[e] = 0.0;
 #pragma unroll
-        for (int j = 0; j < APT; ++j) {
-          const int k = tid + j * kConsumerThreads;
-          if (k < len) {
-            const float x0 = gs[k * 3 + 0], x1 = gs[k * 3 + 1], x2 = gs[k * 3 + 2];
-            const double ty0 = R[0] * yr[j][0] + R[3] * yr[j][1] + R[6] * yr[j][2];
-            const double ty1 = R[1] * yr[j][0] + R[4] * yr[j][1] + R[7] * yr[j][2];
-            const double ty2 = R[2] * yr[j][0] + R[5] * yr[j][1] + R[8] * yr[j][2];
-            gs[k * 3 + 0] = (float)(scale * (((double)x0 - cc[0]) - ty0));
-            gs[k * 3 + 1] = (float)(scale * (((double)x1 - cc[1]) - ty1));
-            gs[k * 3 + 2] = (float)(scale * (((double)x2 - cc[2]) - ty2));
-          }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      }
-      named_barrier_sync(1, kConsumerThreads);
-      // byte range of this item in the gradient array and its aligned middle
-      const uint64_t b0 = (uint64_t)(c.f * sg.n_atoms + a0) * 12ull;
-      const uint64_t b1 = b0 + (uint64_t)len * 12ull;
-      const uint64_t m0 = (b0 + 15ull) & ~15ull, m1 = b1 & ~15ull;
-      const bool mid = m1 > m0;
-      unsigned char* gbase = reinterpret_cast<unsigned char*>(sg.grad);
-      const unsigned char* sbase = reinterpret_cast<const unsigned char*>(gs) - (b0 & 15ull);  // holds byte b0 & ~15
-      if (tid == 0) {
-        if (ok && has_grad && !*abort_flag && mid) {
-          bulk_copy_s2g(gbase + m0, sbase + (m0 - (b0 & ~15ull)), (uint32_t)(m1 - m0));
-        }
-        bulk_commit();
-        // the stage read by the previous item's store is refilled next
-        bulk_wait_read<1>();
-        if (issued < n_items) {
-          const int sp = (int)(issued % S);
-          batched_issue<APT>(B.segs[pc.seg], pc.t, pc.f, smem + sp * G::kStageBytes, &full[sp], rec_src);
-          ++issued;
-          cursor_next(B, pc);
-        }
-      } else if (ok && has_grad && tid >= 32 && tid < 38) {
-        // ends outside the aligned middle: [b0, m0) and [m1, b1), or all of [b0, b1)
-        const int q = tid - 32;  // 0..2 head, 3..5 tail
-        const uint64_t at = mid ? (q < 3 ? b0 + 4ull * q : m1 + 4ull * (q - 3)) : b0 + 4ull * q;
-        const uint64_t lim = mid ? (q < 3 ? m0 : b1) : b1;
-        if (at < lim)
-          *reinterpret_cast<float*>(gbase + at) = *reinterpret_cast<const float*>(sbase + (at - (b0 & ~15ull)));
-      }
-    } else {
-      double acc[16];
+    for (int j = 0; j < APT; ++j) {
+      if ((warp << 5) + j * kConsumerThreads >= len) break;  // warp-uniform: the rest of the tile is empty
+      const int k = tid + j * kConsumerThreads;
+      const bool in = ok && k < len;
+      const double x0 = in ? (double)xs[k * 3 + 0] : 0.0;
+      const double x1 = in ? (double)xs[k * 3 + 1] : 0.0;
+      const double x2 = in ? (double)xs[k * 3 + 2] : 0.0;
+      acc[0] += x0; acc[1] += x1; acc[2] += x2;
+      acc[3] = fma(x0, x0, acc[3]); acc[4] = fma(x1, x1, acc[4]); acc[5] = fma(x2, x2, acc[5]);
+      acc[6] = fma(x0, yr[j][0], acc[6]);  acc[7] = fma(x0, yr[j][1], acc[7]);  acc[8] = fma(x0, yr[j][2], acc[8]);
+      acc[9] = fma(x1, yr[j][0], acc[9]);  acc[10] = fma(x1, yr[j][1], acc[10]); acc[11] = fma(x1, yr[j][2], acc[11]);
+      acc[12] = fma(x2, yr[j][0], acc[12]); acc[13] = fma(x2, yr[j][1], acc[13]); acc[14] = fma(x2, yr[j][2], acc[14]);
+    }
+    const double v = warp_reduce_scatter16(acc);
+    double* rb = red + (i & 1) * (kConsumerWarps * 16);
+    if ((lane & 1) == 0) rb[warp * 16 + (lane >> 1)] = v;
+    named_barrier_sync(1, kConsumerThreads);
+    if (warp == (int)(i & (kConsumerWarps - 1)) && lane < 16) {
+      double tot = 0.0;
 #pragma unroll
-      for (int e = 0; e < 16; ++e) acc[e] = 0.0;
-#pragma unroll
-      for (int j = 0; j < APT; ++j) {
-        if ((warp << 5) + j * kConsumerThreads >= len) break;  // warp-uniform: the rest of the tile is empty
-        const int k = tid + j * kConsumerThreads;
-        const bool in = ok && k < len;
-        const double x0 = in ? (double)xs[k * 3 + 0] : 0.0;
-        const double x1 = in ? (double)xs[k * 3 + 1] : 0.0;
-        const double x2 = in ? (double)xs[k * 3 + 2] : 0.0;
-        acc[0] += x0; acc[1] += x1; acc[2] += x2;
-        acc[3] = fma(x0, x0, acc[3]); acc[4] = fma(x1, x1, acc[4]); acc[5] = fma(x2, x2, acc[5]);
-        acc[6] = fma(x0, yr[j][0], acc[6]);  acc[7] = fma(x0, yr[j][1], acc[7]);  acc[8] = fma(x0, yr[j][2], acc[8]);
-        acc[9] = fma(x1, yr[j][0], acc[9]);  acc[10] = fma(x1, yr[j][1], acc[10]); acc[11] = fma(x1, yr[j][2], acc[11]);
-        acc[12] = fma(x2, yr[j][0], acc[12]); acc[13] = fma(x2, yr[j][1], acc[13]); acc[14] = fma(x2, yr[j][2], acc[14]);
-      }
-      const double v = warp_reduce_scatter16(acc);
-      double* rb = red + (i & 1) * (kConsumerWarps * 16);
-      if ((lane & 1) == 0) rb[warp * 16 + (lane >> 1)] = v;
-      named_barrier_sync(1, kConsumerThreads);
-      if (warp == (int)(i & (kConsumerWarps - 1)) && lane < 16) {
-        double tot = 0.0;
-#pragma unroll
-        for (int wv = 0; wv < kConsumerWarps; ++wv) tot += rb[wv * 16 + lane];
-        B.partial[(size_t)gitem * kStatDoubles + lane] = tot;
-      }
+      for (int wv = 0; wv < kConsumerWarps; ++wv) tot += rb[wv * 16 + lane];
+      B.partial[(size_t)gitem * kStatDoubles + lane] = tot;
     }
     if (*abort_flag) break;
     if (++s == S) { s = 0; phase ^= 1u; }
     cursor_next(B, c);
   }
   if (tid == 0) {
-    if (MODE == kBBwd) bulk_wait_all<0>();
     const int64_t first = issued > S ? issued - S : 0;
     for (int64_t j = first; j < issued; ++j) {
       const int st = (int)(j % S);
@@ -292,6 +229,144 @@ __global__ void __launch_bounds__(kThreads, 4) batched_stream_kernel(const Batch
         }
       }
     }
+  }
+}
+
+// The gradient pass over the same items.  128 threads write dRMSD/dx over x in the
+// stage (each its own atoms) and count themselves done with it on the stage's second
+// mbarrier; a producer warp then stores the tile (one bulk store of its 16-byte-aligned
+// middle, at most 2 x 3 scalar floats at its ends) and refills the stage of the item before
+// once that one's store has read it.  The frame's rotation record comes with its
+// coordinates.  Bound by HBM (24 B per atom-frame) for whole tiles, by a fixed part
+// per item for small ones (the producer's chain): 780 ns up to 64 atoms, 1,250 at 512,
+// 2,466 at 1,024 with 592 CTAs; with a CTA barrier per item and one of the 128 threads
+// storing, waiting and refilling 1,085, 1,440 and 2,500.
+constexpr int kGradThreads = kConsumerThreads + 32;
+
+template <int APT>
+__global__ void __launch_bounds__(kGradThreads, 4) batched_grad_kernel(const BatchLaunch B) {
+  using G = BGeo<APT>;
+  constexpr int T = G::kTile;
+  constexpr int S = G::kStages;
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + G::kBarOffset);
+  uint64_t* ready = reinterpret_cast<uint64_t*>(smem + G::kRedOffset);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + G::kAbortOffset);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int64_t W = B.total_items;
+  const int64_t w0 = W * blockIdx.x / gridDim.x, w1 = W * (blockIdx.x + 1) / gridDim.x;
+  const int64_t n_items = w1 - w0;
+  if (tid == 0) {
+    for (int st = 0; st < S; ++st) {
+      mbar_init(&full[st], 1);
+      mbar_init(&ready[st], kConsumerThreads);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (n_items <= 0) return;
+  Cursor c;
+  cursor_init(B, w0, c);
+  int s = 0;
+  uint32_t phase = 0;
+
+  if (tid >= kConsumerThreads) {
+    // ---------------- producer ----------------
+    Cursor pc = c;
+    int64_t issued = 0;
+    auto issue = [&]() {  // lane 0
+      const int sp = (int)(issued % S);
+      batched_issue<APT>(B.segs[pc.seg], pc.t, pc.f, smem + sp * G::kStageBytes, &full[sp], B.rot);
+      ++issued;
+      cursor_next(B, pc);
+    };
+    if (lane == 0)
+      while (issued < S && issued < n_items) issue();
+    for (int64_t i = 0; i < n_items; ++i) {
+      const BatchSeg& sg = B.segs[c.seg];
+      const int64_t a0 = (int64_t)c.t * T;
+      const int len = (int)(min(sg.n_atoms, a0 + T) - a0);
+      const bool ok = mbar_wait(&ready[s], phase, B.status, kStatusTimeoutEmpty, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      // byte range of this item in the gradient array and its aligned middle
+      const uint64_t b0 = (uint64_t)(c.f * sg.n_atoms + a0) * 12ull, b1 = b0 + (uint64_t)len * 12ull;
+      const uint64_t m0 = (b0 + 15ull) & ~15ull, m1 = b1 & ~15ull;
+      const bool mid = m1 > m0;
+      unsigned char* gbase = reinterpret_cast<unsigned char*>(sg.grad);
+      const unsigned char* sbase = smem + s * G::kStageBytes;  // holds byte b0 & ~15
+      if (gbase && lane < 6) {
+        // ends outside the aligned middle: [b0, m0) and [m1, b1), or all of [b0, b1)
+        const uint64_t at = mid ? (lane < 3 ? b0 + 4ull * lane : m1 + 4ull * (lane - 3)) : b0 + 4ull * lane;
+        const uint64_t lim = mid ? (lane < 3 ? m0 : b1) : b1;
+        if (at < lim)
+          *reinterpret_cast<float*>(gbase + at) = *reinterpret_cast<const float*>(sbase + (at - (b0 & ~15ull)));
+      }
+      __syncwarp();  // the ends are read before the stage is refilled
+      if (lane == 0) {
+        if (gbase && mid) bulk_copy_s2g(gbase + m0, sbase + (m0 - (b0 & ~15ull)), (uint32_t)(m1 - m0));
+        bulk_commit();
+        if (i > 0 && issued < n_items) {
+          bulk_wait_read<1>();  // the previous item's store has read its stage
+          issue();
+        }
+      }
+      if (++s == S) { s = 0; phase ^= 1u; }
+      cursor_next(B, c);
+    }
+    if (lane == 0) {
+      bulk_wait_all<0>();
+      const int64_t first = issued > S ? issued - S : 0;
+      for (int64_t j = first; j < issued; ++j) mbar_drain(&full[j % S], (uint32_t)((j / S) & 1), B.status);
+    }
+    return;
+  }
+
+  // ---------------- consumers ----------------
+  int cur_seg = -1, cur_tile = -1;
+  double yr[APT][3];
+  for (int64_t i = 0; i < n_items; ++i) {
+    const BatchSeg& sg = B.segs[c.seg];
+    const int64_t a0 = (int64_t)c.t * T;
+    const int len = (int)(min(sg.n_atoms, a0 + T) - a0);
+    if (c.seg != cur_seg || c.t != cur_tile) {
+      cur_seg = c.seg;
+      cur_tile = c.t;
+#pragma unroll
+      for (int j = 0; j < APT; ++j) {
+        const int k = tid + j * kConsumerThreads;
+        const double* y = sg.yc + (a0 + k) * 3;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) yr[j][e] = k < len ? y[e] : 0.0;
+      }
+    }
+    if (!mbar_wait(&full[s], phase, B.status, kStatusTimeoutFull, abort_flag)) break;
+    if (sg.grad != nullptr) {
+      float* gs = reinterpret_cast<float*>(smem + s * G::kStageBytes) + (int)(((uint64_t)(c.f * sg.n_atoms + a0) * 3) & 3ull);
+      const double* rt = reinterpret_cast<const double*>(smem + s * G::kStageBytes + G::kRecOffset);
+      double R[9], cc[3];
+#pragma unroll
+      for (int e = 0; e < 9; ++e) R[e] = rt[e];
+      cc[0] = rt[9]; cc[1] = rt[10]; cc[2] = rt[11];
+      const double scale = rt[12];
+#pragma unroll
+      for (int j = 0; j < APT; ++j) {
+        const int k = tid + j * kConsumerThreads;
+        if (k < len) {
+          const float x0 = gs[k * 3 + 0], x1 = gs[k * 3 + 1], x2 = gs[k * 3 + 2];
+          const double ty0 = R[0] * yr[j][0] + R[3] * yr[j][1] + R[6] * yr[j][2];
+          const double ty1 = R[1] * yr[j][0] + R[4] * yr[j][1] + R[7] * yr[j][2];
+          const double ty2 = R[2] * yr[j][0] + R[5] * yr[j][1] + R[8] * yr[j][2];
+          gs[k * 3 + 0] = (float)(scale * (((double)x0 - cc[0]) - ty0));
+          gs[k * 3 + 1] = (float)(scale * (((double)x1 - cc[1]) - ty1));
+          gs[k * 3 + 2] = (float)(scale * (((double)x2 - cc[2]) - ty2));
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    mbar_arrive(&ready[s]);
+    if (++s == S) { s = 0; phase ^= 1u; }
+    cursor_next(B, c);
   }
 }
 
@@ -1253,8 +1328,14 @@ int frame_occupancy() {
 }
 
 template <int APT, int MODE>
+auto stream_kernel() {
+  if constexpr (MODE == kBBwd) return batched_grad_kernel<APT>;
+  else return batched_stream_kernel<APT>;
+}
+
+template <int APT, int MODE>
 cudaError_t launch_stream(const BatchLaunch& B, int grid, cudaStream_t s) {
-  auto kern = batched_stream_kernel<APT, MODE>;
+  auto kern = stream_kernel<APT, MODE>();
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1264,16 +1345,17 @@ cudaError_t launch_stream(const BatchLaunch& B, int grid, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
-  kern<<<grid, kThreads, BGeo<APT>::kSmemBytes, s>>>(B);
+  kern<<<grid, MODE == kBBwd ? kGradThreads : kThreads, BGeo<APT>::kSmemBytes, s>>>(B);
   return cudaGetLastError();
 }
 
 template <int APT, int MODE>
 int occupancy_of() {
-  auto kern = batched_stream_kernel<APT, MODE>;
+  auto kern = stream_kernel<APT, MODE>();
+  const int threads = MODE == kBBwd ? kGradThreads : kThreads;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BGeo<APT>::kSmemBytes);
   int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, kThreads, BGeo<APT>::kSmemBytes) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, threads, BGeo<APT>::kSmemBytes) != cudaSuccess)
     blocks = 1;
   return blocks < 1 ? 1 : blocks;
 }
