@@ -1,7 +1,6 @@
-"""The frames-across-lanes kernel finishing its own frames (a warp finishes the
-32-frame group whose last tile it stored) and summing the frames past the last
-quad row, against the same frames run 16 at a time, which takes the atom-major
-kernel and the finalize kernel.
+"""The frames-across-lanes kernel finishing its own frames (the last warp of a 32-frame
+group to store its sums finishes the group) and summing the frames past the last quad
+row, against the same frames run 16 at a time, which takes other kernels.
 
 Tolerance: both sum in FP64 in different orders, so G and lambda differ by a few
 eps of G (coordinates ~50 A from the origin): 1e-9 A, as the batched tests; an
